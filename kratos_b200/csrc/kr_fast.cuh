@@ -5,7 +5,7 @@
 // reciprocal: 1 / rho per state, 1 / (gamma - 1) and gamma - 1 from the host,
 // rsqrt for the star-state densities, one reciprocal per HLLD star denominator,
 // and the van Leer PLM slope (dl dc / (dl + dc), algebraically the reference's
-// dl dc (dl + dc) / (dl^2 + dc^2 + 2 dl dc)) with one reciprocal for both faces.
+// dl dc (dl + dc) / (dl^2 + dc^2 + 2 dl dc)).
 // Results differ from the reference by rounding only; the GPU parity tests state
 // the bound.  FP64 divides are long dependent DFMA sequences, so this is what
 // moves the FP64 flux kernel off its latency floor.
@@ -20,15 +20,63 @@ template< class R > struct eos_c
     R gamma, gm1, cv;        // gamma, gamma - 1, 1 / (gamma - 1)
 };
 
-// FP64: correctly rounded reciprocal / IEEE square root.  FP32 (the mixed
-// step, whose error budget is 1e-4 in density): the SFU approximations, one
-// MUFU instruction each instead of an IEEE refinement sequence.
-__device__ __forceinline__ double rcp( double x ) { return __drcp_rn( x ); }
-__device__ __forceinline__ float  rcp( float x )  { return __fdividef( 1.0f, x ); }
-__device__ __forceinline__ double rsq( double x ) { return rsqrt( x ); }
-__device__ __forceinline__ float  rsq( float x )  { return rsqrtf( x ); }
-__device__ __forceinline__ double fsqrt( double x ) { return sqrt( x ); }
-__device__ __forceinline__ float  fsqrt( float x )  { return x > 0.f ? x * rsqrtf( x ) : 0.f; }
+// FP32 (the mixed step, whose error budget is 1e-4 in density): the SFU
+// approximations, one MUFU instruction each.  The .ftz forms: without them every
+// reciprocal carries a compare and two scalings for subnormal inputs, which no
+// caller has (densities and pressures are above their floors, the limiter's sums
+// are normal, below).  A subnormal square is taken as zero.
+__device__ __forceinline__ float rcp( float x )
+{
+    float y;
+    asm( "rcp.approx.ftz.f32 %0, %1;" : "=f"( y ) : "f"( x ) );
+    return y;
+}
+__device__ __forceinline__ float rsq( float x )
+{
+    float y;
+    asm( "rsqrt.approx.ftz.f32 %0, %1;" : "=f"( y ) : "f"( x ) );
+    return y;
+}
+__device__ __forceinline__ float fsqrt( float x ) { return x >= FLT_MIN ? x * rsq( x ) : 0.f; }
+// FP64: Newton-Raphson from the hardware's approximations (about 20 bits): two
+// steps y += y ( 1 - x y ) of the reciprocal; for the reciprocal root one step of
+// third order, from e = 1 - x y^2: y ( 1 + e / 2 + 3 e^2 / 8 ), and one of second.
+// Without the library functions' branches for zero, subnormal and infinite
+// arguments, a face's independent reciprocals overlap.
+__device__ __forceinline__ double rcp( double x )
+{
+    double y;
+    asm( "rcp.approx.ftz.f64 %0, %1;" : "=d"( y ) : "d"( x ) );
+    y = fma( y, fma( -x, y, 1.0 ), y );
+    return fma( y, fma( -x, y, 1.0 ), y );
+}
+__device__ __forceinline__ double rsq3( double x )
+{
+    double y;
+    asm( "rsqrt.approx.ftz.f64 %0, %1;" : "=d"( y ) : "d"( x ) );
+    const double e = fma( -x * y, y, 1.0 );
+    return fma( y * e, fma( 0.375, e, 0.5 ), y );
+}
+__device__ __forceinline__ double rsq( double x )
+{
+    const double y = rsq3( x );
+    return fma( 0.5 * y, fma( -x * y, y, 1.0 ), y );
+}
+__device__ __forceinline__ double fsqrt( double x )
+{   // x / sqrt( x ) with one correction of the product
+    const double y = rsq3( x ), g = x * y;
+    return x > 1e-290 ? fma( 0.5 * y, fma( -g, g, x ), g ) : 0.0;
+}
+
+// Limited slope of a cell (half its van Leer difference, plm.h:116-153
+// mathematics), FP64: q + s is its state at the upper face, q - s at the lower.
+__device__ __forceinline__ double plm_slope( double qm, double q, double qp )
+{
+    const double dl = q - qm, dr = qp - q, p = dl * dr;
+    const bool pos = p > 0;
+    const double s = p * rcp( pos ? dl + dr : 1.0 );
+    return pos ? s : 0.0;
+}
 
 // PLM on one face from the four cells around it (plm.h:116-153 mathematics).
 template< class R > __device__ __forceinline__
@@ -53,15 +101,8 @@ void plm_face_fast( R q_ll, R q_l, R q_r, R q_rr, R & ql, R & qr )
         qr = rpos ? q_r - dqr * ( dqc * rcp( dqc + dqr ) ) : q_r;
         return;
     }
-    const R scale = R( 1 );
-    const R dq2_l = dql * dqc;
-    const R dq2_r = dqr * dqc;
-    const bool lpos = dq2_l > 0, rpos = dq2_r > 0;
-    const R sl = lpos ? dql + dqc : R( 1 );
-    const R sr = rpos ? dqc + dqr : R( 1 );
-    const R inv = rcp( sl * sr );
-    ql = lpos ? q_l + dq2_l * sr * inv * scale : q_l;
-    qr = rpos ? q_r - dq2_r * sl * inv * scale : q_r;
+    ql = q_l + plm_slope( q_ll, q_l, q_r );
+    qr = q_r - plm_slope( q_l, q_r, q_rr );
 }
 
 // The FP32 limiter of plm_face_fast on two variables at once (.x, .y): the
@@ -89,18 +130,6 @@ void plm_face_fast2( float2 q_ll, float2 q_l, float2 q_r, float2 q_rr, float2 & 
     const float2 cr = __ffma2_rn( dqr, tr, q_r );        // q_r - dqr ( dqc / ( dqc + dqr ) )
     ql = make_float2( lx ? cl.x : q_l.x, ly ? cl.y : q_l.y );
     qr = make_float2( rx ? cr.x : q_r.x, ry ? cr.y : q_r.y );
-}
-
-// Fast magnetosonic speed from squared field components and 1 / rho.
-template< class R > __device__ __forceinline__
-R c_fms_fast( R pre, R inv_rho, R bn2, R bt2, R gam )
-{
-    const R cs_2  = gam * pre * inv_rho;
-    const R v_ax2 = bn2 * inv_rho;
-    const R v_t2  = bt2 * inv_rho;
-    const R q_2   = v_ax2 + v_t2 + cs_2;
-    const R r_2   = v_ax2 + v_t2 - cs_2;
-    return fsqrt( R( 0.5f ) * ( q_2 + fsqrt( r_2 * r_2 + R( 4 ) * cs_2 * v_t2 ) ) );
 }
 
 ////////////////////////////////////////////////////////////
@@ -171,193 +200,208 @@ void hllc_fast( R * flx, const R * wl, const R * wr, const eos_c< R > & e )
 }
 
 ////////////////////////////////////////////////////////////
-// HLLD on rotated primitive states (hlld.h:81-298 mathematics).
+// HLLD and HLLE on rotated primitive states (hlld.h:31-298 mathematics).
+//
+// The left and right states go through the same arithmetic up to the contact
+// speed and the star states, so they are kept as pairs (.x left, .y right) and
+// FP32 uses sm_100's paired instructions: one issue slot for both sides (the
+// sweep is bound by instruction issue in FP32, by latency in FP64).  The HLLD
+// flux of a star region is the physical flux of its state -- the star states
+// satisfy the jump conditions across the outer and the Alfven waves -- so
+// instead of F + S (U* - U) + ... over eight conserved words of both sides, one
+// side's region state is selected and put through one flux; energies are formed
+// for that side only, and no branch on the contact's side is left.  Where a star
+// state is degenerate (f_tiny below) the reference keeps the outer transverse
+// field, whose jump the contact speed does not satisfy: the field flux then takes
+// the difference B_t (v_n - S_M).
+// Flux sweeps z / y / x of the 256^3 mesh in 64 blocks of 64^3, ms per launch,
+// with the reciprocals above: FP64 1.62 / 1.50 / 1.41 -> 0.67 / 0.65 / 0.58, FP32
+// 0.48 / 0.45 / 0.37 -> 0.35 / 0.33 / 0.31.  FP32 states against FP64 after 6 to
+// 12 steps of a smooth flow: 0.4 to 0.5 of the two-sided form's distance.
 
-template< class R > __device__ __forceinline__
-R hlld_cons_fast( R * u, const R * w, R bx_2, R b_x, const eos_c< R > & e )
-{
-    const R p_m = ( bx_2 + w[ BCC + 1 ] * w[ BCC + 1 ] + w[ BCC + 2 ] * w[ BCC + 2 ] ) * R( 0.5f );
-    const R v2 = w[ MOM ] * w[ MOM ] + w[ MOM + 1 ] * w[ MOM + 1 ] + w[ MOM + 2 ] * w[ MOM + 2 ];
-    u[ RHO ] = w[ RHO ];
-    u[ ENE ] = w[ ENE ] * e.cv + w[ RHO ] * v2 * R( 0.5f ) + p_m;
-    for( int n = MOM; n < MOM + 3; ++ n )
-        u[ n ] = w[ RHO ] * w[ n ];
-    u[ BCC ] = b_x;
-    u[ BCC + 1 ] = w[ BCC + 1 ];
-    u[ BCC + 2 ] = w[ BCC + 2 ];
-    return p_m;
-}
+template< class R > struct lr_t;
+template<> struct lr_t< float >  { typedef float2 type; };
+template<> struct lr_t< double > { typedef double2 type; };
+template< class R > using lr = typename lr_t< R >::type;
 
-template< class R > __device__ __forceinline__
-R hlld_star_fast( R * us, const R * u, const R * w, R rhos, R inv_rhos, R sd, R inv_sdm,
-                  R p_tot, R b_x, R bx_2, R ptot_s, R spd0, R f_tiny, R sdm )
-{
-    us[ RHO ] = rhos;
-    us[ MOM ] = rhos * spd0;
-    us[ BCC ] = b_x;
-    const R denom = u[ RHO ] * sd * sdm - bx_2;
-    if( uabs( denom ) < f_tiny * ptot_s )
-        for( int a = 1; a <= 2; ++ a )
-        {
-            us[ MOM + a ] = rhos * w[ MOM + a ];
-            us[ BCC + a ] = u[ BCC + a ];
-        }
-    else
-    {
-        const R id = rcp( denom );
-        const R tmp_v = b_x * ( sd - sdm ) * id;
-        const R tmp_b = ( u[ RHO ] * sd * sd - bx_2 ) * id;
-        for( int a = 1; a <= 2; ++ a )
-        {
-            us[ MOM + a ] = rhos * ( w[ MOM + a ] - u[ BCC + a ] * tmp_v );
-            us[ BCC + a ] = u[ BCC + a ] * tmp_b;
-        }
-    }
-    R u_dot_b = 0, w_dot_b = 0;
-    for( int a = 0; a < 3; ++ a )
-    {
-        u_dot_b += us[ MOM + a ] * us[ BCC + a ];
-        w_dot_b += w[ MOM + a ] * u[ BCC + a ];
-    }
-    u_dot_b *= inv_rhos;
-    us[ ENE ] = ( b_x * ( w_dot_b - u_dot_b ) - p_tot * w[ MOM ] + sd * u[ ENE ] + ptot_s * spd0 ) * inv_sdm;
-    return u_dot_b;
-}
+__device__ __forceinline__ float2  mk2( float a, float b )   { return make_float2( a, b ); }
+__device__ __forceinline__ double2 mk2( double a, double b ) { return make_double2( a, b ); }
+__device__ __forceinline__ float2 add2( float2 a, float2 b ) { return __fadd2_rn( a, b ); }
+__device__ __forceinline__ float2 mul2( float2 a, float2 b ) { return __fmul2_rn( a, b ); }
+__device__ __forceinline__ float2 mad2( float2 a, float2 b, float2 c ) { return __ffma2_rn( a, b, c ); }
+__device__ __forceinline__ float2 sub2( float2 a, float2 b ) { return __ffma2_rn( b, make_float2( -1.f, -1.f ), a ); }
+__device__ __forceinline__ double2 add2( double2 a, double2 b ) { return make_double2( a.x + b.x, a.y + b.y ); }
+__device__ __forceinline__ double2 mul2( double2 a, double2 b ) { return make_double2( a.x * b.x, a.y * b.y ); }
+__device__ __forceinline__ double2 mad2( double2 a, double2 b, double2 c ) { return make_double2( a.x * b.x + c.x, a.y * b.y + c.y ); }
+__device__ __forceinline__ double2 sub2( double2 a, double2 b ) { return make_double2( a.x - b.x, a.y - b.y ); }
+template< class P > __device__ __forceinline__ P rcp2( P a ) { return mk2( rcp( a.x ), rcp( a.y ) ); }
+template< class P > __device__ __forceinline__ P rsq2( P a ) { return mk2( rsq( a.x ), rsq( a.y ) ); }
+// Square roots of positive pairs
+__device__ __forceinline__ float2 root2( float2 a ) { return mul2( a, rsq2( a ) ); }
+__device__ __forceinline__ double2 root2( double2 a ) { return make_double2( fsqrt( a.x ), fsqrt( a.y ) ); }
 
-// What HLLD and HLLE (the learned mode's cheap flux) both start from: the
-// conserved states, total pressures and the outer wave speeds.
+// What both solvers start from: the states, total pressures and outer speeds.
 template< class R > struct hll_prefix
 {
-    R u_l[ 8 ], u_r[ 8 ];
-    R b_x, bx_2, pm_l, pm_r, spd_m2, spd_p2;
+    lr< R > rho, pre, vn, vt1, vt2, bt1, bt2, pm;
+    R b_x, bx_2, spd_m2, spd_p2;
 };
 
 template< class R > __device__ __forceinline__
 void hll_prefix_fast( hll_prefix< R > & h, const R * wl, const R * wr, const eos_c< R > & e )
 {
+    typedef lr< R > P;
+    const P half = mk2( R( 0.5f ), R( 0.5f ) );
+    h.rho = mk2( wl[ RHO ], wr[ RHO ] );
+    h.pre = mk2( wl[ ENE ], wr[ ENE ] );
+    h.vn  = mk2( wl[ MOM ], wr[ MOM ] );
+    h.vt1 = mk2( wl[ MOM + 1 ], wr[ MOM + 1 ] );
+    h.vt2 = mk2( wl[ MOM + 2 ], wr[ MOM + 2 ] );
+    h.bt1 = mk2( wl[ BCC + 1 ], wr[ BCC + 1 ] );
+    h.bt2 = mk2( wl[ BCC + 2 ], wr[ BCC + 2 ] );
     h.b_x = wl[ BCC ];
     h.bx_2 = h.b_x * h.b_x;
-    h.pm_l = hlld_cons_fast( h.u_l, wl, h.bx_2, h.b_x, e );
-    h.pm_r = hlld_cons_fast( h.u_r, wr, h.bx_2, h.b_x, e );
-    const R irl = rcp( wl[ RHO ] ), irr = rcp( wr[ RHO ] );
-    const R cfm_l = c_fms_fast( wl[ ENE ], irl, h.bx_2,
-                                wl[ BCC + 1 ] * wl[ BCC + 1 ] + wl[ BCC + 2 ] * wl[ BCC + 2 ], e.gamma );
-    const R cfm_r = c_fms_fast( wr[ ENE ], irr, h.bx_2,
-                                wr[ BCC + 1 ] * wr[ BCC + 1 ] + wr[ BCC + 2 ] * wr[ BCC + 2 ], e.gamma );
-    h.spd_m2 = rmin( wl[ MOM ] - cfm_l, wr[ MOM ] - cfm_r );
-    h.spd_p2 = rmax( wl[ MOM ] + cfm_l, wr[ MOM ] + cfm_r );
+    const P b2 = mk2( h.bx_2, h.bx_2 );
+    const P bt = mad2( h.bt1, h.bt1, mul2( h.bt2, h.bt2 ) );
+    h.pm = mul2( half, add2( b2, bt ) );
+    // fast magnetosonic speeds (mhd/eos/adiabatic.h:84-98)
+    const P ir = rcp2( h.rho );
+    const P cs = mul2( mul2( mk2( e.gamma, e.gamma ), h.pre ), ir );
+    const P vt = mul2( bt, ir ), va = mul2( b2, ir );
+    const P s = add2( va, vt ), q = add2( s, cs ), r = sub2( s, cs );
+    P rad = mad2( r, r, mul2( mul2( mk2( R( 4 ), R( 4 ) ), cs ), vt ) );
+    const R tiny = sizeof( R ) == 4 ? R( FLT_MIN ) : R( 1e-290 );
+    rad = mk2( rmax( rad.x, tiny ), rmax( rad.y, tiny ) );       // its root: finite at zero
+    const P cf = root2( mul2( half, mad2( rad, rsq2( rad ), q ) ) );
+    const P sm = sub2( h.vn, cf ), sp = add2( h.vn, cf );
+    h.spd_m2 = rmin( sm.x, sm.y );
+    h.spd_p2 = rmax( sp.x, sp.y );
 }
 
-// HLLD from the prefix (mhd/riemann/hlld.h:31-298).
 template< class R > __device__ __forceinline__
-void hlld_tail( R * flx, const R * wl, const R * wr, const hll_prefix< R > & h )
+void hlld_tail( R * flx, const hll_prefix< R > & h, const eos_c< R > & e )
 {
-    const R * u_l = h.u_l, * u_r = h.u_r;
-    const R b_x = h.b_x, bx_2 = h.bx_2, spd_m2 = h.spd_m2, spd_p2 = h.spd_p2;
-    const R ptot_l = wl[ ENE ] + h.pm_l, ptot_r = wr[ ENE ] + h.pm_r;
-    flx[ BCC ] = 0;
-    if( spd_m2 >= 0 || spd_p2 <= 0 )
-    {
-        const bool is_left = spd_m2 >= 0;
-        hlld_f_flux( flx, is_left ? u_l : u_r, is_left ? wl : wr, is_left ? ptot_l : ptot_r, b_x );
-        flx[ BCC ] = 0;
-        return;
-    }
-    const R sd_l = spd_m2 - wl[ MOM ];
-    const R sd_r = spd_p2 - wr[ MOM ];
-    const R spd0 = ( sd_r * u_r[ MOM ] - ptot_r - sd_l * u_l[ MOM ] + ptot_l )
-                 * rcp( sd_r * u_r[ RHO ] - sd_l * u_l[ RHO ] );
-    const R sdm_l = spd_m2 - spd0, sdm_r = spd_p2 - spd0;
-    const R isdm = rcp( sdm_l * sdm_r );
-    const R inv_sdm_l = sdm_r * isdm, inv_sdm_r = sdm_l * isdm;
-    const R rhos_l = u_l[ RHO ] * sd_l * inv_sdm_l;
-    const R rhos_r = u_r[ RHO ] * sd_r * inv_sdm_r;
-    const R rs_l = rsq( rhos_l ), rs_r = rsq( rhos_r );       // 1 / sqrt(rho*)
-    const R rhos_l_sqrt = rhos_l * rs_l, rhos_r_sqrt = rhos_r * rs_r;
-    const R irs_l = rs_l * rs_l, irs_r = rs_r * rs_r;          // 1 / rho*
-    const R spd_m1 = spd0 - uabs( b_x ) * rs_l;
-    const R spd_p1 = spd0 + uabs( b_x ) * rs_r;
+    typedef lr< R > P;
+    const R b_x = h.b_x, bx_2 = h.bx_2;
     const R f_tiny = R( 1.00e-4f );
-    const R ptot_s = ptot_l + u_l[ RHO ] * sd_l * ( sd_l - sdm_l );
-    R us_l[ 8 ], us_r[ 8 ];
-    const R udb_l = hlld_star_fast( us_l, u_l, wl, rhos_l, irs_l, sd_l, inv_sdm_l, ptot_l,
-                                    b_x, bx_2, ptot_s, spd0, f_tiny, sdm_l );
-    const R udb_r = hlld_star_fast( us_r, u_r, wr, rhos_r, irs_r, sd_r, inv_sdm_r, ptot_r,
-                                    b_x, bx_2, ptot_s, spd0, f_tiny, sdm_r );
-    if( spd_m1 >= 0 )
-    {
-        hlld_f_flux( flx, u_l, wl, ptot_l, b_x );
-        for( int n = 0; n < 8; ++ n )
-            flx[ n ] += spd_m2 * ( us_l[ n ] - u_l[ n ] );
-        flx[ BCC ] = 0;
-        return;
-    }
-    if( spd_p1 <= 0 )
-    {
-        hlld_f_flux( flx, u_r, wr, ptot_r, b_x );
-        for( int n = 0; n < 8; ++ n )
-            flx[ n ] += spd_p2 * ( us_r[ n ] - u_r[ n ] );
-        flx[ BCC ] = 0;
-        return;
-    }
-    R uss_l[ 8 ], uss_r[ 8 ];
-    for( int n = 0; n < 8; ++ n )
-    {
-        uss_l[ n ] = us_l[ n ];
-        uss_r[ n ] = us_r[ n ];
-    }
-    if( bx_2 > ptot_s * f_tiny )
-    {
-        const R bx_sgn = b_x > 0 ? R( 1 ) : R( -1 );
-        const R rni = rcp( rhos_l_sqrt + rhos_r_sqrt );
-        for( int a = 1; a <= 2; ++ a )
-        {
-            R tmp = rni * ( us_l[ MOM + a ] * rs_l + us_r[ MOM + a ] * rs_r
-                          + bx_sgn * ( us_r[ BCC + a ] - us_l[ BCC + a ] ) );
-            uss_l[ MOM + a ] = uss_l[ RHO ] * tmp;
-            uss_r[ MOM + a ] = uss_r[ RHO ] * tmp;
-            tmp = rni * ( rhos_l_sqrt * us_r[ BCC + a ] + rhos_r_sqrt * us_l[ BCC + a ]
-                        + bx_sgn * rhos_l_sqrt * rhos_r_sqrt
-                        * ( us_r[ MOM + a ] * irs_r - us_l[ MOM + a ] * irs_l ) );
-            uss_l[ BCC + a ] = tmp;
-            uss_r[ BCC + a ] = tmp;
-        }
-        const R tmp = spd0 * b_x + ( uss_l[ MOM + 1 ] * uss_l[ BCC + 1 ]
-                                   + uss_l[ MOM + 2 ] * uss_l[ BCC + 2 ] ) * irs_l;
-        uss_l[ ENE ] -= rhos_l_sqrt * bx_sgn * ( udb_l - tmp );
-        uss_r[ ENE ] += rhos_r_sqrt * bx_sgn * ( udb_r - tmp );
-    }
-    if( spd0 >= 0 )
-    {
-        hlld_f_flux( flx, u_l, wl, ptot_l, b_x );
-        const R d_v = spd_m1 - spd_m2;
-        for( int n = 0; n < 8; ++ n )
-            flx[ n ] += -spd_m2 * u_l[ n ] - d_v * us_l[ n ] + spd_m1 * uss_l[ n ];
-    }
+    const P nb2 = mk2( -bx_2, -bx_2 ), bx = mk2( b_x, b_x );
+    const P pt = add2( h.pre, h.pm );
+    const P s2 = mk2( h.spd_m2, h.spd_p2 );
+    const P sd = sub2( s2, h.vn );
+    const P m = mul2( h.rho, sd );                              // rho ( S - v_n )
+    const P u_m = mul2( h.rho, h.vn );
+    const R spd0 = ( sd.y * u_m.y - pt.y - sd.x * u_m.x + pt.x ) * rcp( m.y - m.x );
+    const P s0 = mk2( spd0, spd0 );
+    const P sdm = sub2( s2, s0 ), dv = sub2( h.vn, s0 );
+    const R ptot_s = pt.x - m.x * dv.x;
+    P ism;
+    if constexpr( sizeof( R ) == 4 )
+        ism = rcp2( sdm );
     else
-    {
-        hlld_f_flux( flx, u_r, wr, ptot_r, b_x );
-        const R d_v = spd_p1 - spd_p2;
-        for( int n = 0; n < 8; ++ n )
-            flx[ n ] += -spd_p2 * u_r[ n ] - d_v * us_r[ n ] + spd_p1 * uss_r[ n ];
+    {   // one reciprocal for both sides
+        const R i = rcp( sdm.x * sdm.y );
+        ism = mk2( sdm.y * i, sdm.x * i );
     }
+    const P rhos = mul2( m, ism );
+    const P rs = rsq2( rhos );                                  // 1 / sqrt( rho* )
+    const P sq = mul2( rhos, rs );
+    const P denom = mad2( m, sdm, nb2 );
+    const P id = rcp2( denom );
+    P tv = mul2( mul2( bx, dv ), id );
+    P tb = mul2( mad2( m, sd, nb2 ), id );
+    const R flat = f_tiny * ptot_s;
+    const bool flat_l = uabs( denom.x ) < flat, flat_r = uabs( denom.y ) < flat;
+    tv = mk2( flat_l ? R( 0 ) : tv.x, flat_r ? R( 0 ) : tv.y );
+    tb = mk2( flat_l ? R( 1 ) : tb.x, flat_r ? R( 1 ) : tb.y );
+    const P vs1 = mad2( h.bt1, tv, h.vt1 ), vs2 = mad2( h.bt2, tv, h.vt2 );
+    const P bs1 = mul2( h.bt1, tb ), bs2 = mul2( h.bt2, tb );
+    const R spd_m1 = spd0 - uabs( b_x ) * rs.x, spd_p1 = spd0 + uabs( b_x ) * rs.y;
+    // the side the face lies on, and whether outside its fan, in its star or
+    // in its double-star region
+    const bool out_l = h.spd_m2 >= 0, out_r = h.spd_p2 <= 0, outer = out_l || out_r;
+    const bool left = out_l || ( ! out_r && spd0 >= 0 );
+    const bool inner = ! outer && ( left ? spd_m1 < 0 : spd_p1 > 0 ) && bx_2 > flat;
+    R rho = left ? h.rho.x : h.rho.y, vn = left ? h.vn.x : h.vn.y, p = left ? pt.x : pt.y;
+    R v1 = left ? h.vt1.x : h.vt1.y, v2 = left ? h.vt2.x : h.vt2.y;
+    R b1 = left ? h.bt1.x : h.bt1.y, bb2 = left ? h.bt2.x : h.bt2.y;
+    const R pre = left ? h.pre.x : h.pre.y, pm = left ? h.pm.x : h.pm.y;
+    R en = pre * e.cv + rho * ( vn * vn + v1 * v1 + v2 * v2 ) * R( 0.5f ) + pm;
+    R vb = vn * b_x + v1 * b1 + v2 * bb2;
+    R x1 = 0, x2 = 0, mass = left ? u_m.x : u_m.y;
+    if( ! outer )
+    {
+        const R sdl = left ? sd.x : sd.y, il = left ? ism.x : ism.y;
+        const bool flt = left ? flat_l : flat_r;
+        const R dvn = vn - spd0;
+        x1 = flt ? b1 * dvn : R( 0 );
+        x2 = flt ? bb2 * dvn : R( 0 );
+        const R rho_s = left ? rhos.x : rhos.y;
+        if constexpr( sizeof( R ) == 8 )
+        {   // FP64: the mass flux as the sum of its jumps.  Against a wall it is
+            // rounding residue, whose sign the edge EMF's upwind switch reads:
+            // the region's rho S_M is exactly zero there, which the reference's
+            // sum is not
+            const R so = left ? h.spd_m2 : h.spd_p2, si = left ? spd_m1 : spd_p1;
+            mass += ( left ? si < 0 : si > 0 ) ? - so * rho - ( si - so ) * rho_s + si * rho_s
+                                               : so * ( rho_s - rho );
+        }
+        else
+            mass = rho_s * spd0;
+        rho = rho_s;
+        v1 = left ? vs1.x : vs1.y; v2 = left ? vs2.x : vs2.y;
+        b1 = left ? bs1.x : bs1.y; bb2 = left ? bs2.x : bs2.y;
+        const R vbs = spd0 * b_x + v1 * b1 + v2 * bb2;
+        en = ( b_x * ( vb - vbs ) - p * vn + sdl * en + ptot_s * spd0 ) * il;
+        vb = vbs;
+        vn = spd0;
+        p = ptot_s;
+        if( inner )
+        {
+            const R sg = b_x > 0 ? R( 1 ) : R( -1 );
+            const R rni = rcp( sq.x + sq.y ), ss = sg * sq.x * sq.y;
+            v1 = rni * ( sq.x * vs1.x + sq.y * vs1.y + sg * ( bs1.y - bs1.x ) );
+            v2 = rni * ( sq.x * vs2.x + sq.y * vs2.y + sg * ( bs2.y - bs2.x ) );
+            b1 = rni * ( sq.x * bs1.y + sq.y * bs1.x + ss * ( vs1.y - vs1.x ) );
+            bb2 = rni * ( sq.x * bs2.y + sq.y * bs2.x + ss * ( vs2.y - vs2.x ) );
+            const R vbd = spd0 * b_x + v1 * b1 + v2 * bb2;
+            en += ( left ? -sq.x : sq.y ) * sg * ( vb - vbd );
+            vb = vbd;
+        }
+    }
+    const R mn = rho * vn;
+    flx[ RHO ] = mass;
+    flx[ ENE ] = ( en + p ) * vn - b_x * vb;
+    flx[ MOM ] = mn * vn + p - bx_2;
+    flx[ MOM + 1 ] = mn * v1 - b_x * b1;
+    flx[ MOM + 2 ] = mn * v2 - b_x * bb2;
     flx[ BCC ] = 0;
+    flx[ BCC + 1 ] = b1 * vn - b_x * v1 + x1;
+    flx[ BCC + 2 ] = bb2 * vn - b_x * v2 + x2;
 }
 
 // HLLE with the HLLD outer speeds, from the prefix.
 template< class R > __device__ __forceinline__
-void hlle_tail( R * flx, const R * wl, const R * wr, const hll_prefix< R > & h )
+void hlle_tail( R * flx, const hll_prefix< R > & h, const eos_c< R > & e )
 {
-    R f_l[ 8 ], f_r[ 8 ];
+    typedef lr< R > P;
     const R s_l = rmin( h.spd_m2, R( 0 ) );
     const R s_r = rmax( h.spd_p2, R( 0 ) );
-    hlld_f_flux( f_l, h.u_l, wl, wl[ ENE ] + h.pm_l, h.b_x );
-    hlld_f_flux( f_r, h.u_r, wr, wr[ ENE ] + h.pm_r, h.b_x );
-    f_l[ BCC ] = f_r[ BCC ] = 0;
-    const R inv = rcp( s_r - s_l );
-    for( int n = 0; n < 8; ++ n )
-        flx[ n ] = ( s_r * f_l[ n ] - s_l * f_r[ n ] + s_r * s_l * ( h.u_r[ n ] - h.u_l[ n ] ) ) * inv;
+    const R inv = rcp( s_r - s_l ), slr = s_r * s_l;
+    const P bx = mk2( h.b_x, h.b_x ), half = mk2( R( 0.5f ), R( 0.5f ) );
+    const P mn = mul2( h.rho, h.vn );
+    const P v2 = mad2( h.vn, h.vn, mad2( h.vt1, h.vt1, mul2( h.vt2, h.vt2 ) ) );
+    const P en = mad2( h.pre, mk2( e.cv, e.cv ), mad2( mul2( half, h.rho ), v2, h.pm ) );
+    const P pt = sub2( add2( h.pre, h.pm ), mk2( h.bx_2, h.bx_2 ) );
+    const P vb = mad2( h.vt1, h.bt1, mul2( h.vt2, h.bt2 ) );
+    auto join = [ & ]( P f, P u ) { return ( s_r * f.x - s_l * f.y + slr * ( u.y - u.x ) ) * inv; };
+    flx[ RHO ] = join( mn, h.rho );
+    flx[ ENE ] = join( sub2( mul2( h.vn, add2( pt, en ) ), mul2( bx, vb ) ), en );
+    flx[ MOM ] = join( mad2( mn, h.vn, pt ), mn );
+    flx[ MOM + 1 ] = join( sub2( mul2( mn, h.vt1 ), mul2( bx, h.bt1 ) ), mul2( h.rho, h.vt1 ) );
+    flx[ MOM + 2 ] = join( sub2( mul2( mn, h.vt2 ), mul2( bx, h.bt2 ) ), mul2( h.rho, h.vt2 ) );
     flx[ BCC ] = 0;
+    flx[ BCC + 1 ] = join( sub2( mul2( h.bt1, h.vn ), mul2( bx, h.vt1 ) ), h.bt1 );
+    flx[ BCC + 2 ] = join( sub2( mul2( h.bt2, h.vn ), mul2( bx, h.vt2 ) ), h.bt2 );
 }
 
 template< class R > __device__ __forceinline__
@@ -365,7 +409,7 @@ void hlld_fast( R * flx, const R * wl, const R * wr, const eos_c< R > & e )
 {
     hll_prefix< R > h;
     hll_prefix_fast( h, wl, wr, e );
-    hlld_tail( flx, wl, wr, h );
+    hlld_tail( flx, h, e );
 }
 
 // HLLE with the HLLD outer speeds (cheap flux of the learned selector).
@@ -374,7 +418,7 @@ void hlle_fast( R * flx, const R * wl, const R * wr, const eos_c< R > & e )
 {
     hll_prefix< R > h;
     hll_prefix_fast( h, wl, wr, e );
-    hlle_tail( flx, wl, wr, h );
+    hlle_tail( flx, h, e );
 }
 
 // The learned mode's solver of one face, HLLE where `cheap`, else HLLD, from
@@ -384,8 +428,8 @@ void hll_pick_fast( R * flx, const R * wl, const R * wr, const eos_c< R > & e, b
 {
     hll_prefix< R > h;
     hll_prefix_fast( h, wl, wr, e );
-    if( cheap ) hlle_tail( flx, wl, wr, h );
-    else        hlld_tail( flx, wl, wr, h );
+    if( cheap ) hlle_tail( flx, h, e );
+    else        hlld_tail( flx, h, e );
 }
 
 }   // namespace kr
