@@ -3,7 +3,7 @@
 //
 // Every kernel kind of the step runs as ONE persistent launch whose CTAs walk
 // a work list: one item per CTA tile that the per-group launches would run
-// (group, block, z plane, tile along the plane), bigger blocks first.  A CTA
+// (group, block, plane or row of planes, tile along it), bigger blocks first.  A CTA
 // takes items blockIdx.x, blockIdx.x + gridDim.x, ... and runs the same
 // per-site code on the item's group arguments (read from the kernel's
 // parameter space by the item's group index), so a batched step gives the
@@ -26,24 +26,20 @@ template< class R >
 struct multi_t
 {
     args_t< R > a[ KR_BATCH_MAX ];
-    udiv_t dv_c[ KR_BATCH_MAX ];          // c2p rows: n0
-    udiv_t dv_e[ KR_BATCH_MAX ];          // edge / lattice rows: n0 + 1
+    tile_t cells[ KR_BATCH_MAX ];         // a block's cells
+    tile_t lattice[ KR_BATCH_MAX ];       // and its edge / lattice sites
     udiv_t dv_f[ 3 ][ KR_BATCH_MAX ];     // face rows of each sweep
     unsigned cpp_f[ 3 ][ KR_BATCH_MAX ];  // 128-face tiles per z plane of each sweep
-    // the work lists [c2p | flux z | flux y | flux x | lattice sites]: per list,
+    // the work lists [cells | flux z | flux y | flux x | lattice sites]: per list,
     // the first item of each group in list order (l_off[.][ng] = the count),
-    // that group, and its tiles per plane and planes per block
+    // that group, and its tiles per plane (cells, lattice: per row of planes)
+    // and planes per block
     int ng;
     int l_off[ 5 ][ KR_BATCH_MAX + 1 ];
     int l_grp[ 5 ][ KR_BATCH_MAX ];
     udiv_t l_tiles[ 5 ][ KR_BATCH_MAX ];   // multiply-high quotients (d = 1: the identity)
     udiv_t l_planes[ 5 ][ KR_BATCH_MAX ];
 };
-
-__device__ __forceinline__ unsigned udiv_q1( unsigned n, const udiv_t & v )
-{
-    return v.d == 1 ? n : udiv_q( n, v );
-}
 
 // Item it of work list `list`: x group, y block, z plane, w tile.  Uniform over
 // the CTA when it is (it comes from blockIdx and the loop counter).
@@ -101,7 +97,7 @@ k_c2p_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
         const int4 t = batch_item( m, 0, it );
-        c2p_cells< MHD, R, DT >( m.a[ t.x ], step, m.dv_c[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
+        c2p_cells< MHD, R, DT >( m.a[ t.x ], step, m.cells[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
         if( DT )
             __syncthreads(  );            // the CTA reduction's shared words are reused
     }
@@ -146,7 +142,7 @@ k_emf_list( const __grid_constant__ multi_t< R > m, int n_items )
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
         const int4 t = batch_item( m, 4, it );
-        emf_site< R >( m.a[ t.x ], m.dv_e[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
+        emf_site< R >( m.a[ t.x ], m.lattice[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
     }
 }
 
@@ -156,8 +152,8 @@ k_update_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
 {
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
-        const int4 t = batch_item( m, 4, it );
-        update_site< MHD, R, false, PART >( m.a[ t.x ], step, m.dv_e[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
+        const int4 t = batch_item( m, PART == 1 ? 0 : 4, it );
+        update_site< MHD, R, false, PART >( m.a[ t.x ], step, PART == 1 ? m.cells[ t.x ] : m.lattice[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
     }
 }
 
@@ -170,12 +166,9 @@ k_update_c2p_list( const __grid_constant__ multi_t< R > m, int n_items )
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
         const int4 t = batch_item( m, 0, it );
-        const args_t< R > & a = m.a[ t.x ];
-        const unsigned c = unsigned( t.w ) * 256u + threadIdx.x;
-        if( c >= unsigned( a.n0 * a.n1 ) )
-            continue;
-        const unsigned q = udiv_q( c, m.dv_c[ t.x ] );
-        update_c2p_cell< R >( a, t.y, int( c - q * unsigned( a.n0 ) ), int( q ), t.z );
+        int i[ 3 ];
+        if( tile_site( m.cells[ t.x ], t.z, unsigned( t.w ) * 256u + threadIdx.x, i ) )
+            update_c2p_cell< R >( m.a[ t.x ], t.y, i[ 0 ], i[ 1 ], i[ 2 ] );
     }
 }
 
@@ -204,7 +197,7 @@ struct kr_batch
     std::vector< kr_ctx * > ctx;
     std::string err;
     int precision = 2, riemann = 0;
-    // work lists: [c2p | flux z | flux y | flux x | lattice sites], ordered
+    // work lists: [cells | flux z | flux y | flux x | lattice sites], ordered
     // bigger blocks first (decoded on the device, batch_item)
     long long cnt[ 5 ] = { 0 };
     int l_off[ 5 ][ KR_BATCH_MAX + 1 ] = { { 0 } }, l_grp[ 5 ][ KR_BATCH_MAX ] = { { 0 } };
@@ -237,8 +230,8 @@ static multi_t< R > make_multi( kr_batch * bt )
         kr_ctx * c = bt->ctx[ g ];
         const int * n = c->cfg.n;
         m.a[ g ] = make_args< R >( c );
-        m.dv_c[ g ] = make_udiv( unsigned( n[ 0 ] ) );
-        m.dv_e[ g ] = make_udiv( unsigned( n[ 0 ] + 1 ) );
+        m.cells[ g ] = make_tile( n[ 0 ], n[ 1 ], n[ 2 ] );
+        m.lattice[ g ] = make_tile( n[ 0 ] + 1, n[ 1 ] + 1, n[ 2 ] + 1 );
         for( int axis = 0; axis < 3; ++ axis )
         {
             int ext[ 3 ];
@@ -321,7 +314,7 @@ static void batch_enqueue( kr_batch * bt, cudaStream_t st, T && timed )
                 k_update_c2p_list< R ><<< bgrid( bt, BK_UPDC2P, 0 ), 256, 0, st >>>( m, int( bt->cnt[ 0 ] ) ); } );
             continue;
         }
-        timed( BK_UPD1, [ & ] { k_update_list< true, R, 1 ><<< bgrid( bt, BK_UPD1, 4 ), 256, 0, st >>>( m, stage, ne ); } );
+        timed( BK_UPD1, [ & ] { k_update_list< true, R, 1 ><<< bgrid( bt, BK_UPD1, 0 ), 256, 0, st >>>( m, stage, int( bt->cnt[ 0 ] ) ); } );
         timed( BK_UPD2, [ & ] { k_update_list< true, R, 2 ><<< bgrid( bt, BK_UPD2, 4 ), 256, 0, st >>>( m, stage, ne ); } );
     }
     k_step_end_multi<<< 1, 1, 0, st >>>( ms, bt->ctx[ 0 ]->cfg.dt_expand );
@@ -502,8 +495,13 @@ kr_batch * kr_batch_create( kr_ctx * const * ctxs, int n )
             const int g = order[ p ];
             const int * nn = ctxs[ g ]->cfg.n;
             long long tiles, planes;
-            if( list == 0 )      { tiles = blocks_for( ( long long ) nn[ 0 ] * nn[ 1 ], 256 ); planes = nn[ 2 ]; }
-            else if( list == 4 ) { tiles = blocks_for( ( long long )( nn[ 0 ] + 1 ) * ( nn[ 1 ] + 1 ), 256 ); planes = nn[ 2 ] + 1; }
+            if( list == 0 || list == 4 )
+            {
+                const int e = list == 4;
+                const tile_t t = make_tile( nn[ 0 ] + e, nn[ 1 ] + e, nn[ 2 ] + e );
+                tiles = tile_ctas( t );
+                planes = tile_rows( t );
+            }
             else
             {
                 const int axis = 2 - ( list - 1 );

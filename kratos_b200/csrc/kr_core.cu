@@ -149,6 +149,44 @@ static inline udiv_t make_udiv( unsigned d )
 }
 __device__ __forceinline__ unsigned udiv_q( unsigned n, const udiv_t & v ) { return __umulhi( n, v.m ); }
 
+__device__ __forceinline__ unsigned udiv_q1( unsigned n, const udiv_t & v )   // d >= 1
+{
+    return v.d == 1 ? n : udiv_q( n, v );
+}
+
+// The sites of a block (e0 x e1 x e2, x fastest) over CTAs of 256 threads: a
+// row of CTAs walks `g` planes as one index, so small planes share CTAs (the
+// 17 x 17 edge sites of a 16^3 block's plane filled 56% of two CTAs, its 17
+// planes fill 96% of 20).  g: all planes, or as many as keep the quotients exact.
+struct tile_t
+{
+    int e0, e1, e2, g;
+    udiv_t d0, d01;
+};
+static inline tile_t make_tile( int e0, int e1, int e2 )
+{
+    const long long p = ( long long ) e0 * e1;
+    const long long most = std::max( 1LL, std::min< long long >( e2, ( ( 1LL << 32 ) - 1 ) / ( p * p ) ) );
+    const long long rows = ( e2 + most - 1 ) / most;
+    return { e0, e1, e2, int( ( e2 + rows - 1 ) / rows ), make_udiv( unsigned( e0 ) ), make_udiv( unsigned( p ) ) };
+}
+static inline unsigned tile_ctas( const tile_t & t )
+{
+    return unsigned( ( ( long long ) t.e0 * t.e1 * t.g + 255 ) / 256 );
+}
+static inline unsigned tile_rows( const tile_t & t ) { return unsigned( ( t.e2 + t.g - 1 ) / t.g ); }
+
+// Site s of row `row`; false past the block's last site.
+__device__ __forceinline__ bool tile_site( const tile_t & t, int row, unsigned s, int * i )
+{
+    const unsigned p = t.g == 1 ? 0u : udiv_q( s, t.d01 ), r = s - p * t.d01.d;
+    const unsigned q = udiv_q( r, t.d0 );
+    i[ 0 ] = int( r - q * t.d0.d );
+    i[ 1 ] = int( q );
+    i[ 2 ] = row * t.g + int( p );
+    return i[ 1 ] < t.e1 && int( p ) < t.g && i[ 2 ] < t.e2;
+}
+
 __device__ __forceinline__ double warp_min( double v )
 {
     for( int o = 16; o > 0; o >>= 1 )
@@ -273,17 +311,16 @@ void c2p_point( const args_t< R > & a, R * W, double * U, int b, int i0, int i1,
 
 // DT: stage 0's launch, which also reduces the CFL dt; stage 1's launch has none
 // of that code (fewer registers).
-// One CTA's cells: block b, z plane i2, cell c of the (x, y) plane (every
-// thread of the CTA calls it: the dt reduction is CTA-wide).
+// One CTA's cells: block b, site c of row `row` of its cells (every thread of
+// the CTA calls it: the dt reduction is CTA-wide).
 template< bool MHD, class R, bool DT > __device__ __forceinline__
-void c2p_cells( const args_t< R > & a, int step, udiv_t dv, int b, int i2, unsigned c )
+void c2p_cells( const args_t< R > & a, int step, const tile_t & tl, int b, int row, unsigned c )
 {
     double dt = FLT_MAX;
-    if( c < unsigned( a.n0 * a.n1 ) )
+    int ic[ 3 ];
+    if( tile_site( tl, row, c, ic ) )
     {
-        const unsigned q = udiv_q( c, dv );
-        const int i0 = int( c - q * unsigned( a.n0 ) );
-        const int i1 = int( q );
+        const int i0 = ic[ 0 ], i1 = ic[ 1 ], i2 = ic[ 2 ];
         double * U = a.u[ step ];
         double cons[ 5 ], prim[ 5 ];
         for( int k = 0; k < 5; ++ k )
@@ -357,10 +394,10 @@ void c2p_cells( const args_t< R > & a, int step, udiv_t dv, int b, int i2, unsig
 }
 
 template< bool MHD, class R, bool DT >
-__global__ void __launch_bounds__( 256, ( MHD && DT ) ? 3 : 4 ) k_c2p( const args_t< R > a, int step, udiv_t dv )
+__global__ void __launch_bounds__( 256, ( MHD && DT ) ? 3 : 4 ) k_c2p( const args_t< R > a, int step, tile_t tl )
 {
-    // grid: x over the cells of one (x, y) plane, y over z, z over blocks
-    c2p_cells< MHD, R, DT >( a, step, dv, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
+    // grid: x, y over the block's cells (tile_t), z over blocks
+    c2p_cells< MHD, R, DT >( a, step, tl, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
 }
 
 ////////////////////////////////////////////////////////////
@@ -1202,15 +1239,13 @@ R face_emf( const args_t< R > & a, int b, int fa, int ax, const int * i )
     return a.f[ fa ][ ifx( a, b, slot, 7, i[ 0 ], i[ 1 ], i[ 2 ] ) ];
 }
 
-// Edge site t of the (x, y) plane i2 of block b.
+// Edge site t of row `row` of block b.
 template< class R > __device__ __forceinline__
-void emf_site( const args_t< R > & a, udiv_t dv, int b, int i2, unsigned t )
+void emf_site( const args_t< R > & a, const tile_t & tl, int b, int row, unsigned t )
 {
-    const int e0 = a.n0 + 1, e1 = a.n1 + 1;
-    if( t >= unsigned( e0 * e1 ) )
+    int i[ 3 ];
+    if( ! tile_site( tl, row, t, i ) )
         return;
-    const unsigned q = udiv_q( t, dv );
-    int i[ 3 ] = { int( t - q * unsigned( e0 ) ), int( q ), i2 };
     const int nn[ 3 ] = { a.n0, a.n1, a.n2 };
     const R w_e = R( 0.25f );
     // one base offset per site (cell E in W, the fluxes, the edge EMF); the
@@ -1281,10 +1316,10 @@ void emf_site( const args_t< R > & a, udiv_t dv, int b, int i2, unsigned t )
 }
 
 template< class R >
-__global__ void __launch_bounds__( 256 ) k_emf( const args_t< R > a, udiv_t dv )
+__global__ void __launch_bounds__( 256 ) k_emf( const args_t< R > a, tile_t tl )
 {
-    // grid: x over the edges of one (x, y) plane, y over z, z over blocks
-    emf_site< R >( a, dv, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
+    // grid: x, y over the block's edge sites (tile_t), z over blocks
+    emf_site< R >( a, tl, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
 }
 
 ////////////////////////////////////////////////////////////
@@ -1451,18 +1486,16 @@ double ct_face( const args_t< R > & a, const geo_t & g, int b, int c, const int 
     return nb;
 }
 
-// PART 0: cells and faces in one launch; 1: the conserved update only; 2: the
-// CT face update only (MHD: two launches, each with fewer registers).
-// Lattice site t of the (x, y) plane i2 of block b.
+// PART 1: the conserved update of the cells; 2 (MHD): the CT update of the faces
+// (two launches, each with fewer registers).  Site t of row `row` of block b: a
+// cell, or a lattice site (its three lower faces).
 template< bool MHD, class R, bool SMR, int PART > __device__ __forceinline__
-void update_site( const args_t< R > & a, int step, udiv_t dv, int b, int i2, unsigned t )
+void update_site( const args_t< R > & a, int step, const tile_t & tl, int b, int row, unsigned t )
 {
     constexpr int NF = MHD ? 7 : 5;
-    const int e0 = a.n0 + 1, e1 = a.n1 + 1;
-    if( t >= unsigned( e0 * e1 ) )
+    int i[ 3 ];
+    if( ! tile_site( tl, row, t, i ) )
         return;
-    const unsigned q = udiv_q( t, dv );
-    int i[ 3 ] = { int( t - q * unsigned( e0 ) ), int( q ), i2 };
     const int nn[ 3 ] = { a.n0, a.n1, a.n2 };
     // Heun: U* = U + dt L(U), U' = (U + U*) / 2 + dt / 2 L(U*); VL2:
     // U* = U + dt / 2 L1(U), U' = U + dt L(U*)
@@ -1473,7 +1506,7 @@ void update_site( const args_t< R > & a, int step, udiv_t dv, int b, int i2, uns
     // issue ahead of the stores of earlier ones.
     const R * __restrict__ F[ 3 ] = { a.f[ 0 ], a.f[ 1 ], a.f[ 2 ] };
     const R * __restrict__ EE = a.ee;
-    if( PART != 2 && i[ 0 ] < nn[ 0 ] && i[ 1 ] < nn[ 1 ] && i[ 2 ] < nn[ 2 ] )
+    if( PART == 1 )
     {
         const double * __restrict__ us = a.u[ step ];
         double * __restrict__ ut = a.u[ 1 - step ];
@@ -1599,11 +1632,11 @@ void update_site( const args_t< R > & a, int step, udiv_t dv, int b, int i2, uns
     }
 }
 
-template< bool MHD, class R, bool SMR = false, int PART = 0 >
-__global__ void __launch_bounds__( 256, ( SMR && sizeof( R ) == 4 ) ? 4 : ( PART == 2 ? 6 : 4 ) ) k_update( const args_t< R > a, int step, udiv_t dv )
+template< bool MHD, class R, bool SMR, int PART >
+__global__ void __launch_bounds__( 256, ( SMR && sizeof( R ) == 4 ) ? 4 : ( PART == 2 ? 6 : 4 ) ) k_update( const args_t< R > a, int step, tile_t tl )
 {
-    // grid: x over the lattice sites of one (x, y) plane, y over z, z over blocks
-    update_site< MHD, R, SMR, PART >( a, step, dv, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
+    // grid: x, y over the block's cells or lattice sites (tile_t), z over blocks
+    update_site< MHD, R, SMR, PART >( a, step, tl, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
 }
 
 ////////////////////////////////////////////////////////////
@@ -1657,14 +1690,12 @@ void update_c2p_cell( const args_t< R > & a, int b, int i0, int i1, int i2 )
 }
 
 template< class R >
-__global__ void __launch_bounds__( 256, 4 ) k_update_c2p( const args_t< R > a, udiv_t dv )
+__global__ void __launch_bounds__( 256, 4 ) k_update_c2p( const args_t< R > a, tile_t tl )
 {
-    // grid: x over the cells of one (x, y) plane, y over z, z over blocks
-    const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
-    if( c >= unsigned( a.n0 * a.n1 ) )
-        return;
-    const unsigned q = udiv_q( c, dv );
-    update_c2p_cell< R >( a, blockIdx.z, int( c - q * unsigned( a.n0 ) ), int( q ), blockIdx.y );
+    // grid: x, y over the block's cells (tile_t), z over blocks
+    int i[ 3 ];
+    if( tile_site( tl, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x, i ) )
+        update_c2p_cell< R >( a, blockIdx.z, i[ 0 ], i[ 1 ], i[ 2 ] );
 }
 
 template< bool MHD, class R >
@@ -2267,6 +2298,8 @@ static void launch_flux_mode( kr_ctx * c, cudaStream_t st, const args_t< R > & a
     else                                          launch_flux< MHD, R, KR_RIEMANN_DEFAULT >( c, st, a, axis, stage );
 }
 
+static dim3 tile_grid( const tile_t & t, unsigned nblk ) { return dim3( tile_ctas( t ), tile_rows( t ), nblk ); }
+
 // One stage is front (cons -> prim, CFL dt at stage 0, pack of the halo other
 // ranks read), exchange (NCCL send / receive by peer; at stage 0 the dt
 // all-reduce), back (unpack, same-rank ghosts, physical sides, flux sweeps,
@@ -2287,9 +2320,10 @@ static void enqueue_front( kr_ctx * c, cudaStream_t st, const args_t< R > & a, i
 {
     const unsigned nb = unsigned( c->nblk );
     const int * n = c->cfg.n;
+    const tile_t cells = make_tile( n[ 0 ], n[ 1 ], n[ 2 ] );
     if( ! ( c->fuse && stage == 1 ) )        // (fused: stage 0's update did stage 1's c2p)
-        timed( 0, [ & ] { ( stage == 0 ? k_c2p< MHD, R, true > : k_c2p< MHD, R, false > )<<< dim3( blocks_for( ( long long ) n[ 0 ] * n[ 1 ], 256 ), n[ 2 ], nb ), 256, 0, st >>>(
-            a, stage, make_udiv( unsigned( n[ 0 ] ) ) ); } );
+        timed( 0, [ & ] { ( stage == 0 ? k_c2p< MHD, R, true > : k_c2p< MHD, R, false > )<<< tile_grid( cells, nb ), 256, 0, st >>>(
+            a, stage, cells ); } );
     if( ! c->hsend.items.empty(  ) )
         timed( 1, [ & ] {
             k_halo< MHD, R, true ><<< dim3( c->halo_grid, unsigned( c->hsend.items.size(  ) ) ), 256, 0, st >>>(
@@ -2349,12 +2383,12 @@ static void enqueue_back( kr_ctx * c, cudaStream_t st, const args_t< R > & a, in
                     const long long rows = ( long long )( n[ ( ax + 1 ) % 3 ] + 4 ) * ( n[ ( ax + 2 ) % 3 ] + 4 );
                     k_phys_mhd< R ><<< dim3( blocks_for( rows, 128 ), nb ), 128, 0, st >>>( a, side, stage );
                 } } );
+    const tile_t cells = make_tile( n[ 0 ], n[ 1 ], n[ 2 ] ), lattice = make_tile( n[ 0 ] + 1, n[ 1 ] + 1, n[ 2 ] + 1 );
+    const dim3 gc = tile_grid( cells, nb ), gl = tile_grid( lattice, nb );
     for( int axis = 2; axis >= 0; -- axis )
         timed( 4 - axis, [ & ] { launch_flux_mode< MHD, R >( c, st, a, axis, stage, mode ); } );
     if( MHD )
-        timed( 5, [ & ] { k_emf< R ><<< dim3( blocks_for( ( long long )( n[ 0 ] + 1 ) * ( n[ 1 ] + 1 ), 256 ), n[ 2 ] + 1, nb ), 256, 0, st >>>(
-            a, make_udiv( unsigned( n[ 0 ] + 1 ) ) ); } );
-    const dim3 ug( blocks_for( ( long long )( n[ 0 ] + 1 ) * ( n[ 1 ] + 1 ), 256 ), n[ 2 ] + 1, nb );
+        timed( 5, [ & ] { k_emf< R ><<< gl, 256, 0, st >>>( a, lattice ); } );
     if constexpr( MHD )
         if( c->smr )
         {   // refined MHD (dynamics.h:80-99): the coarse face flux over a
@@ -2364,8 +2398,8 @@ static void enqueue_back( kr_ctx * c, cudaStream_t st, const args_t< R > & a, in
                     k_flux_avg< R, 7 ><<< dim3( blocks_for( smr_half_sites( c ), 128 ), c->n_restrict ), 128, 0, st >>>( a, c->smr_items );
                 for( size_t w = 0; w + 1 < c->mh_waves.size(  ); ++ w )
                     launch_mh< R, MH_FLUX >( c, st, a, c->mh_waves[ w ], c->mh_waves[ w + 1 ], stage );
-                k_update< MHD, R, true, 1 ><<< ug, 256, 0, st >>>( a, stage, make_udiv( unsigned( n[ 0 ] + 1 ) ) );
-                k_update< MHD, R, false, 2 ><<< ug, 256, 0, st >>>( a, stage, make_udiv( unsigned( n[ 0 ] + 1 ) ) ); } );
+                k_update< MHD, R, true, 1 ><<< gc, 256, 0, st >>>( a, stage, cells );
+                k_update< MHD, R, false, 2 ><<< gl, 256, 0, st >>>( a, stage, lattice ); } );
             return;
         }
     if constexpr( ! MHD )
@@ -2374,20 +2408,19 @@ static void enqueue_back( kr_ctx * c, cudaStream_t st, const args_t< R > & a, in
             timed( 6, [ & ] {
                 if( c->n_restrict )      // coarse face flux over a refined side
                     k_flux_avg< R ><<< dim3( blocks_for( smr_half_sites( c ), 128 ), c->n_restrict ), 128, 0, st >>>( a, c->smr_items );
-                k_update< MHD, R, true ><<< ug, 256, 0, st >>>( a, stage, make_udiv( unsigned( n[ 0 ] + 1 ) ) ); } );
+                k_update< MHD, R, true, 1 ><<< gc, 256, 0, st >>>( a, stage, cells ); } );
             return;
         }
     timed( 6, [ & ] {
         if( MHD && c->fuse && stage == 0 )      // update, CT and stage 1's c2p
-            k_update_c2p< R ><<< dim3( blocks_for( ( long long ) n[ 0 ] * n[ 1 ], 256 ), n[ 2 ], nb ), 256, 0, st >>>(
-                a, make_udiv( unsigned( n[ 0 ] ) ) );
+            k_update_c2p< R ><<< gc, 256, 0, st >>>( a, cells );
         else if( MHD )
         {
-            k_update< MHD, R, false, 1 ><<< ug, 256, 0, st >>>( a, stage, make_udiv( unsigned( n[ 0 ] + 1 ) ) );
-            k_update< MHD, R, false, 2 ><<< ug, 256, 0, st >>>( a, stage, make_udiv( unsigned( n[ 0 ] + 1 ) ) );
+            k_update< MHD, R, false, 1 ><<< gc, 256, 0, st >>>( a, stage, cells );
+            k_update< MHD, R, false, 2 ><<< gl, 256, 0, st >>>( a, stage, lattice );
         }
         else
-            k_update< MHD, R ><<< ug, 256, 0, st >>>( a, stage, make_udiv( unsigned( n[ 0 ] + 1 ) ) ); } );
+            k_update< MHD, R, false, 1 ><<< gc, 256, 0, st >>>( a, stage, cells ); } );
 }
 
 // Halo transfer of one stage between this rank and its peers, and at stage 0
