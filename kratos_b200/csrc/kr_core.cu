@@ -6,7 +6,9 @@
 // consecutive x, so all global traffic is coalesced):
 //   U [slot][block][5][n2][n1][n0]           conserved rho, E, m0..2 (double)
 //   BF[slot][block][3][n2+5][n1+5][n0+5]     face B, 2 ghost layers (double)
-//   W [block][nw][n2+4][n1+4][n0+4]          primitives, 2 ghost layers (R)
+//   W [block][nw][n2+4][n1+4][n0+4]          primitives, 2 ghost layers (R); the
+//                                            first 8 (hydro: 4) words of a cell in
+//                                            groups of 16 bytes (w_group)
 //   F [axis][block][nf][n2+3][n1+3][n0+3]    face fluxes, 1 ghost layer (R);
 //                                            nf = 5 hydro, 7 MHD (5 + edge E)
 //   EE[block][3][n2+3][n1+3][n0+3]           edge EMF (R)
@@ -118,10 +120,64 @@ struct args_t
     scal_t * s;
 };
 
+// W keeps the words of a cell that its readers need together in 16-byte groups
+// (FP32: rho p v0 v1 | v2 b0 b1 b2; FP64: pairs; hydro: its first four words),
+// one group array after the other, then the remaining words (MHD: cell E; hydro:
+// v2) as planes: c2p stores a cell with 5 (FP32 MHD) instead of 11 stores, each
+// filling whole lines, and pushes it into a neighbour's ghost shell the same way,
+// and a face's stencil is 8 (FP32) or 16 (FP64) loads instead of 32 or 28.  Per
+// step on 256^3 (64 blocks of 64^3): c2p FP32 1062 -> 860 us, FP64 800 -> 635,
+// FP64 sweeps 3790 -> 3640 (with the normal B's load ahead of the stencil's);
+// refined blast, c2p and level jumps 2990 -> 2050 us.  The FP32 sweeps, bound by
+// issue, got slower (1980 -> 2145: fewer, longer requests leave more of a warp's
+// wait exposed); groups of 8 bytes cost more than they gave (c2p 938).
+template< class R > __host__ __device__ constexpr int w_group(  ) { return 16 / int( sizeof( R ) ); }
+template< bool MHD > __host__ __device__ constexpr int w_grouped(  ) { return MHD ? 8 : 4; }
+template< class R > struct w_vec;
+template<> struct w_vec< float >  { typedef float4 type; };
+template<> struct w_vec< double > { typedef double2 type; };
+
+// Position of cell i in a plane of W, and the index of word c.
+template< class R > __device__ __forceinline__
+int w_pos( const args_t< R > & a, int i0, int i1, int i2 )
+{
+    return ( i0 + 2 ) + a.sw1 * ( i1 + 2 ) + a.sw2 * ( i2 + 2 );
+}
 template< class R > __device__ __forceinline__
 long long iw( const args_t< R > & a, int b, int c, int nw, int i0, int i1, int i2 )
 {
-    return ( long long )( b * nw + c ) * a.ngw + ( i0 + 2 ) + a.sw1 * ( i1 + 2 ) + a.sw2 * ( i2 + 2 );
+    constexpr int G = w_group< R >(  );
+    const long long blk = ( long long ) b * nw * a.ngw;
+    const int pos = w_pos( a, i0, i1, i2 );
+    if( c < ( nw == 11 ? w_grouped< true >(  ) : w_grouped< false >(  ) ) )
+        return blk + ( long long )( c / G * G ) * a.ngw + ( long long ) pos * G + c % G;
+    return blk + ( long long ) c * a.ngw + pos;
+}
+
+// All words of a cell: from / to position pos of block base w.
+template< bool MHD, class R > __device__ __forceinline__
+void w_load( const R * w, long long ngw, int pos, R * v )
+{
+    constexpr int G = w_group< R >(  ), NW = MHD ? 11 : 5, NG = w_grouped< MHD >(  );
+    typedef typename w_vec< R >::type V;
+#pragma unroll
+    for( int k = 0; k < NG; k += G )
+        * reinterpret_cast< V * >( v + k ) = reinterpret_cast< const V * >( w + k * ngw )[ pos ];
+#pragma unroll
+    for( int k = NG; k < NW; ++ k )
+        v[ k ] = w[ k * ngw + pos ];
+}
+template< bool MHD, class R > __device__ __forceinline__
+void w_store( R * w, long long ngw, int pos, const R * v )
+{
+    constexpr int G = w_group< R >(  ), NW = MHD ? 11 : 5, NG = w_grouped< MHD >(  );
+    typedef typename w_vec< R >::type V;
+#pragma unroll
+    for( int k = 0; k < NG; k += G )
+        reinterpret_cast< V * >( w + k * ngw )[ pos ] = * reinterpret_cast< const V * >( v + k );
+#pragma unroll
+    for( int k = NG; k < NW; ++ k )
+        w[ k * ngw + pos ] = v[ k ];
 }
 template< class R > __device__ __forceinline__
 long long iuc( const args_t< R > & a, int b, int c, int i0, int i1, int i2 )
@@ -263,7 +319,7 @@ void c2p_point( const args_t< R > & a, R * W, double * U, int b, int i0, int i1,
         U[ iuc( a, b, ENE, i0, i1, i2 ) ] = MHD ? cout[ ENE ] + e_m : cout[ ENE ];
         atomicAdd( & a.s->heal_count, 1 );
     }
-    R wv[ NW ];
+    alignas( 16 ) R wv[ NW ];
     for( int k = 0; k < 5; ++ k )
         wv[ k ] = R( prim[ k ] );
     if( MHD )
@@ -274,13 +330,7 @@ void c2p_point( const args_t< R > & a, R * W, double * U, int b, int i0, int i1,
             wv[ BCC + d ] = R( bc[ d ] );
             wv[ 8 + d ] = R( bc[ d1 ] ) * R( prim[ MOM + d2 ] ) - R( bc[ d2 ] ) * R( prim[ MOM + d1 ] );
         }
-    const int ngw = int( a.ngw );
-    {
-        R * o = W + iw( a, b, 0, NW, i0, i1, i2 );
-#pragma unroll
-        for( int k = 0; k < NW; ++ k )
-            o[ k * ngw ] = wv[ k ];
-    }
+    w_store< MHD, R >( W + ( size_t ) b * NW * a.ngw, a.ngw, w_pos( a, i0, i1, i2 ), wv );
     // Same-level ghost fill by push: a cell within two cells of a side is a
     // ghost cell of the block across it (faces, edges, corners).  The block
     // that holds this cell's position at i + sh n in its ghost shell is the
@@ -302,10 +352,8 @@ void c2p_point( const args_t< R > & a, R * W, double * U, int b, int i0, int i1,
             const int dst = a.nbr[ b * 27 + ( 1 - dx ) + 3 * ( 1 - dy ) + 9 * ( 1 - dz ) ];
             if( dst < 0 )
                 continue;
-            R * o = W + iw( a, dst, 0, NW, i0 + dx * a.n0, i1 + dy * a.n1, i2 + dz * a.n2 );
-#pragma unroll
-            for( int k = 0; k < NW; ++ k )
-                o[ k * ngw ] = wv[ k ];
+            w_store< MHD, R >( W + ( size_t ) dst * NW * a.ngw, a.ngw,
+                               w_pos( a, i0 + dx * a.n0, i1 + dy * a.n1, i2 + dz * a.n2 ), wv );
         }
 }
 
@@ -515,14 +563,9 @@ __global__ void __launch_bounds__( 256 ) k_ghost( const args_t< R > a, int step,
         const int src = a.nbr[ b * 27 + ( s0 + 1 ) + 3 * ( s1 + 1 ) + 9 * ( s2 + 1 ) ];
         if( src < 0 )
             return;                              // physical side or another rank
-        const int ngw = int( a.ngw );
-        R * dst = a.w + ( size_t ) b * NW * a.ngw + ( ( i0 + 2 ) + a.sw1 * ( i1 + 2 ) + a.sw2 * ( i2 + 2 ) );
-        const R * srcp = a.w + ( size_t ) src * NW * a.ngw + ( ( j0 + 2 ) + a.sw1 * ( j1 + 2 ) + a.sw2 * ( j2 + 2 ) );
-        R v[ NW ];
-        for( int k = 0; k < NW; ++ k )
-            v[ k ] = srcp[ k * ngw ];
-        for( int k = 0; k < NW; ++ k )
-            dst[ k * ngw ] = v[ k ];
+        alignas( 16 ) R v[ NW ];
+        w_load< MHD, R >( a.w + ( size_t ) src * NW * a.ngw, a.ngw, w_pos( a, j0, j1, j2 ), v );
+        w_store< MHD, R >( a.w + ( size_t ) b * NW * a.ngw, a.ngw, w_pos( a, i0, i1, i2 ), v );
         return;
     }
     if( ! MHD )
@@ -1036,17 +1079,13 @@ template< class R, int MODE > constexpr int flux_min_ctas(  )
                             : ( MODE == KR_RIEMANN_HLLE ? 5 : 4 );
 }
 
-// PLM of the NP primitive words of one face from the four cells around it
-// (wb: the right cell's first word, st: stride along the sweep, ngw: word
-// stride); the normal B of an MHD face comes from the face lattice instead.
-// FP32: words k and k + NP / 2 in pairs (plm_face_fast2).
 // The normal B of a face for the reconstruction: the face lattice's value;
 // on a refined MHD mesh, along a transverse ghost line next to a side whose
 // neighbours are on another level, the cell-centred B of the cell above the
 // face instead (mhd/integrator/data.h:98-130 load_primative; no holder
-// carries face B onto those lines).  wb: that cell's first W word.
+// carries face B onto those lines).
 template< class R, bool XL > __device__ __forceinline__
-R normal_b( const args_t< R > & a, int b, int axis, int step, const int * ii, const R * wb )
+R normal_b( const args_t< R > & a, int b, int axis, int step, const int * ii )
 {
     if constexpr( XL )
     {
@@ -1062,60 +1101,80 @@ R normal_b( const args_t< R > & a, int b, int axis, int step, const int * ii, co
                 cross |= ( x >> ( 2 * t + 1 ) ) & 1;
         }
         if( cross )
-            return wb[ ( BCC + axis ) * a.ngw ];
+            return a.w[ iw( a, b, BCC + axis, 11, ii[ 0 ], ii[ 1 ], ii[ 2 ] ) ];
     }
     return R( a.bf[ step ][ ibf( a, b, axis, ii[ 0 ], ii[ 1 ], ii[ 2 ] ) ] );
 }
 
+// PLM of the NP primitive words of one face (ii: its right cell) from the four
+// cells around it (st: stride along the sweep), a 16-byte group of words at a
+// time, FP32 in pairs (plm_face_fast2); the normal B of an MHD face comes from
+// the face lattice instead.
 template< bool MHD, class R, bool XL = false > __device__ __forceinline__
-void plm_stencil( const args_t< R > & a, int b, int axis, int step, const int * ii, const R * wb,
-                  int st, R * ql, R * qr )
+void plm_stencil( const args_t< R > & a, int b, int axis, int step, const int * ii, int st, R * ql, R * qr )
 {
-    constexpr int NP = MHD ? 8 : 5;
-    const int ngw = int( a.ngw );
+    constexpr int NP = MHD ? 8 : 5, NG = w_grouped< MHD >(  ), G = w_group< R >(  ), NW = MHD ? 11 : 5;
+    typedef typename w_vec< R >::type V;
+    const R * w = a.w + ( size_t ) b * NW * a.ngw;
+    const int pos = w_pos( a, ii[ 0 ], ii[ 1 ], ii[ 2 ] );
+    R bn = 0;
+    if constexpr( MHD )
+        bn = normal_b< R, XL >( a, b, axis, step, ii );
     if( a.vl2 && step == 0 )
     {   // VL2 predictor: piecewise-constant (donor-cell) states
-        for( int k = 0; k < NP; ++ k )
+#pragma unroll
+        for( int k = 0; k < NG; k += G )
         {
-            const R * p = wb + k * ngw;
-            ql[ k ] = p[ -st ];
-            qr[ k ] = p[ 0 ];
+            const V * p = reinterpret_cast< const V * >( w + k * a.ngw ) + pos;
+            const V l = p[ -st ], r = p[ 0 ];
+            const R * x = reinterpret_cast< const R * >( & l ), * y = reinterpret_cast< const R * >( & r );
+#pragma unroll
+            for( int g = 0; g < G; ++ g )
+            {
+                ql[ k + g ] = x[ g ];
+                qr[ k + g ] = y[ g ];
+            }
         }
-        if constexpr( MHD )
-            ql[ BCC + axis ] = qr[ BCC + axis ] = normal_b< R, XL >( a, b, axis, step, ii, wb );
-        return;
-    }
-    if constexpr( sizeof( R ) == 4 )
-    {
-        constexpr int H = NP / 2;
-        for( int k = 0; k < H; ++ k )
+        if constexpr( NP > NG )
         {
-            const R * p = wb + k * ngw, * p2 = wb + ( k + H ) * ngw;
-            float2 l2, r2;
-            plm_face_fast2( make_float2( p[ -2 * st ], p2[ -2 * st ] ), make_float2( p[ -st ], p2[ -st ] ),
-                            make_float2( p[ 0 ], p2[ 0 ] ), make_float2( p[ st ], p2[ st ] ), l2, r2 );
-            ql[ k ] = l2.x; ql[ k + H ] = l2.y;
-            qr[ k ] = r2.x; qr[ k + H ] = r2.y;
+            const R * p = w + NG * a.ngw + pos;
+            ql[ NG ] = p[ -st ];
+            qr[ NG ] = p[ 0 ];
         }
-        if constexpr( NP % 2 )
-        {
-            const R * p = wb + ( NP - 1 ) * ngw;
-            plm_face_fast< R >( p[ -2 * st ], p[ -st ], p[ 0 ], p[ st ], ql[ NP - 1 ], qr[ NP - 1 ] );
-        }
-        if constexpr( MHD )
-            ql[ BCC + axis ] = qr[ BCC + axis ] = normal_b< R, XL >( a, b, axis, step, ii, wb );
     }
     else
-        for( int k = 0; k < NP; ++ k )
+    {
+#pragma unroll
+        for( int k = 0; k < NG; k += G )
         {
-            if( MHD && k == BCC + axis )
+            const V * p = reinterpret_cast< const V * >( w + k * a.ngw ) + pos;
+            const V c0 = p[ -2 * st ], c1 = p[ -st ], c2 = p[ 0 ], c3 = p[ st ];
+            if constexpr( sizeof( R ) == 4 )
             {
-                ql[ k ] = qr[ k ] = normal_b< R, XL >( a, b, axis, step, ii, wb );
-                continue;
+                float2 l, r;
+                plm_face_fast2( make_float2( c0.x, c0.y ), make_float2( c1.x, c1.y ),
+                                make_float2( c2.x, c2.y ), make_float2( c3.x, c3.y ), l, r );
+                ql[ k ] = l.x; ql[ k + 1 ] = l.y; qr[ k ] = r.x; qr[ k + 1 ] = r.y;
+                plm_face_fast2( make_float2( c0.z, c0.w ), make_float2( c1.z, c1.w ),
+                                make_float2( c2.z, c2.w ), make_float2( c3.z, c3.w ), l, r );
+                ql[ k + 2 ] = l.x; ql[ k + 3 ] = l.y; qr[ k + 2 ] = r.x; qr[ k + 3 ] = r.y;
             }
-            const R * p = wb + k * ngw;
-            plm_face_fast< R >( p[ -2 * st ], p[ -st ], p[ 0 ], p[ st ], ql[ k ], qr[ k ] );
+            else
+            {
+                if( ! MHD || k != BCC + axis )
+                    plm_face_fast< R >( c0.x, c1.x, c2.x, c3.x, ql[ k ], qr[ k ] );
+                if( ! MHD || k + 1 != BCC + axis )
+                    plm_face_fast< R >( c0.y, c1.y, c2.y, c3.y, ql[ k + 1 ], qr[ k + 1 ] );
+            }
         }
+        if constexpr( NP > NG )
+        {
+            const R * p = w + NG * a.ngw + pos;
+            plm_face_fast< R >( p[ -2 * st ], p[ -st ], p[ 0 ], p[ st ], ql[ NG ], qr[ NG ] );
+        }
+    }
+    if constexpr( MHD )
+        ql[ BCC + axis ] = qr[ BCC + axis ] = bn;
 }
 
 // One CTA's 128 faces of a sweep: bx = CTA along the faces of one (x, y)
@@ -1125,7 +1184,6 @@ template< bool MHD, class R, int MODE, bool XL = false > __device__ __forceinlin
 void flux_faces( const args_t< R > & a, int axis, int step, udiv_t dv, int b, unsigned bx, unsigned by,
                  bool hlle_warp = false )
 {
-    constexpr int NW = MHD ? 11 : 5;   // stored W words: prim (8) + cell E (3)
     constexpr bool learned = MHD && MODE == KR_RIEMANN_LEARNED;
     const int nn[ 3 ] = { a.n0, a.n1, a.n2 };
     unsigned t = bx * blockDim.x + threadIdx.x;
@@ -1168,11 +1226,7 @@ void flux_faces( const args_t< R > & a, int axis, int step, udiv_t dv, int b, un
     const int st = axis == 0 ? 1 : ( axis == 1 ? a.sw1 : a.sw2 );
     R ql[ 8 ], qr[ 8 ];
     if( valid )
-    {
-        const R * wb = a.w + ( size_t ) b * NW * a.ngw
-                     + ( ( ii[ 0 ] + 2 ) + a.sw1 * ( ii[ 1 ] + 2 ) + a.sw2 * ( ii[ 2 ] + 2 ) );
-        plm_stencil< MHD, R, XL >( a, b, axis, step, ii, wb, st, ql, qr );
-    }
+        plm_stencil< MHD, R, XL >( a, b, axis, step, ii, st, ql, qr );
     if constexpr( learned || MODE == FLUX_APPLY )
     {
         if constexpr( learned )
@@ -2887,7 +2941,7 @@ static kr_ctx * create_ctx( const kr_cfg * cfg, int n_regions, const kr_region *
     c->nws = cfg->mhd ? 11 : 5;
     c->nf = cfg->mhd ? 7 : 5;
     c->nc  = ( long long ) n[ 0 ] * n[ 1 ] * n[ 2 ];
-    c->ngw = ( long long )( n[ 0 ] + 4 ) * ( n[ 1 ] + 4 ) * ( n[ 2 ] + 4 );
+    c->ngw = ( ( long long )( n[ 0 ] + 4 ) * ( n[ 1 ] + 4 ) * ( n[ 2 ] + 4 ) + 3 ) & ~ 3LL;   // whole 16-byte groups
     c->nbf = ( long long )( n[ 0 ] + 5 ) * ( n[ 1 ] + 5 ) * ( n[ 2 ] + 5 );
     c->nfb = ( long long )( n[ 0 ] + 3 ) * ( n[ 1 ] + 3 ) * ( n[ 2 ] + 3 );
     c->rsize = cfg->precision == 1 ? 4 : 8;
