@@ -20,7 +20,7 @@
 
 namespace kr
 {
-constexpr int KR_BATCH_MAX = 6;
+constexpr int KR_BATCH_MAX = 6, KR_BATCH_LISTS = 7;
 
 template< class R >
 struct multi_t
@@ -28,17 +28,20 @@ struct multi_t
     args_t< R > a[ KR_BATCH_MAX ];
     tile_t cells[ KR_BATCH_MAX ];         // a block's cells
     tile_t lattice[ KR_BATCH_MAX ];       // and its edge / lattice sites
-    udiv_t dv_f[ 3 ][ KR_BATCH_MAX ];     // face rows of each sweep
-    unsigned cpp_f[ 3 ][ KR_BATCH_MAX ];  // 128-face tiles per z plane of each sweep
-    // the work lists [cells | flux z | flux y | flux x | lattice sites]: per list,
+    udiv_t dv_f[ 3 ][ KR_BATCH_MAX ];     // rows of each sweep's planes
+    unsigned cpp_f[ 3 ][ KR_BATCH_MAX ];  // 128-face tiles per plane of each sweep
+    unsigned warps_f[ 3 ][ KR_BATCH_MAX ];// the march: warps per plane
+    int seg_f[ 3 ][ KR_BATCH_MAX ];       // and faces per segment
+    // the work lists [cells | flux z | flux y | flux x | lattice sites | the z and
+    // y marches]: per list,
     // the first item of each group in list order (l_off[.][ng] = the count),
     // that group, and its tiles per plane (cells, lattice: per row of planes)
     // and planes per block
     int ng;
-    int l_off[ 5 ][ KR_BATCH_MAX + 1 ];
-    int l_grp[ 5 ][ KR_BATCH_MAX ];
-    udiv_t l_tiles[ 5 ][ KR_BATCH_MAX ];   // multiply-high quotients (d = 1: the identity)
-    udiv_t l_planes[ 5 ][ KR_BATCH_MAX ];
+    int l_off[ KR_BATCH_LISTS ][ KR_BATCH_MAX + 1 ];
+    int l_grp[ KR_BATCH_LISTS ][ KR_BATCH_MAX ];
+    udiv_t l_tiles[ KR_BATCH_LISTS ][ KR_BATCH_MAX ];   // multiply-high quotients (d = 1: the identity)
+    udiv_t l_planes[ KR_BATCH_LISTS ][ KR_BATCH_MAX ];
 };
 
 // Item it of work list `list`: x group, y block, z plane, w tile.  Uniform over
@@ -135,6 +138,22 @@ k_flux_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
     }
 }
 
+// The y and z sweeps of a batch that marches (march_pays).
+template< class R, int MODE, int AXIS >
+__global__ void __launch_bounds__( 128, ( march_ctas< R >(  ) ) )
+k_march_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
+{
+    if constexpr( MODE == FLUX_APPLY )
+        if( step == 0 && sel_eval_step( m.a[ 0 ].s, m.a[ 0 ].sel_period ) )
+            return;
+    for( int it = blockIdx.x; it < n_items; it += gridDim.x )
+    {
+        const int4 t = batch_item( m, 7 - AXIS, it );
+        march_tile< R, MODE, false, AXIS >( m.a[ t.x ], step, m.dv_f[ AXIS ][ t.x ], m.warps_f[ AXIS ][ t.x ],
+                                            m.seg_f[ AXIS ][ t.x ], t.y, unsigned( t.w ) );
+    }
+}
+
 template< class R >
 __global__ void __launch_bounds__( 256 )
 k_emf_list( const __grid_constant__ multi_t< R > m, int n_items )
@@ -199,9 +218,11 @@ struct kr_batch
     int precision = 2, riemann = 0;
     // work lists: [cells | flux z | flux y | flux x | lattice sites], ordered
     // bigger blocks first (decoded on the device, batch_item)
-    long long cnt[ 5 ] = { 0 };
-    int l_off[ 5 ][ KR_BATCH_MAX + 1 ] = { { 0 } }, l_grp[ 5 ][ KR_BATCH_MAX ] = { { 0 } };
-    kr::udiv_t l_tiles[ 5 ][ KR_BATCH_MAX ] = { }, l_planes[ 5 ][ KR_BATCH_MAX ] = { };
+    long long cnt[ kr::KR_BATCH_LISTS ] = { 0 };
+    int l_off[ kr::KR_BATCH_LISTS ][ kr::KR_BATCH_MAX + 1 ] = { { 0 } }, l_grp[ kr::KR_BATCH_LISTS ][ kr::KR_BATCH_MAX ] = { { 0 } };
+    kr::udiv_t l_tiles[ kr::KR_BATCH_LISTS ][ kr::KR_BATCH_MAX ] = { }, l_planes[ kr::KR_BATCH_LISTS ][ kr::KR_BATCH_MAX ] = { };
+    kr::march_t shape[ 3 ][ kr::KR_BATCH_MAX ] = { };   // the march, per axis (y, z) and group
+    bool march[ 3 ] = { false, false, false };           // per axis
     bool fuse = false;                   // every context fuses stage 0's update with stage 1's c2p
     int grid[ kr::BK_N ] = { 0 };        // CTAs per launch kind (0: one per item)
     cudaGraph_t graph = nullptr;
@@ -218,6 +239,11 @@ static bool bck( kr_batch * b, cudaError_t e, const char * what )
     if( e == cudaSuccess ) return true;
     b->err = std::string( what ) + ": " + cudaGetErrorString( e );
     return false;
+}
+
+static int batch_plane_axis( const kr_batch * bt, int axis )
+{
+    return bt->riemann == KR_RIEMANN_LEARNED ? face_plane_axis< KR_RIEMANN_LEARNED >( axis ) : face_plane_axis< KR_RIEMANN_DEFAULT >( axis );
 }
 
 template< class R >
@@ -237,8 +263,11 @@ static multi_t< R > make_multi( kr_batch * bt )
             int ext[ 3 ];
             for( int d = 0; d < 3; ++ d )
                 ext[ d ] = ( d == axis ) ? n[ d ] + 1 : n[ d ] + 2;
+            const int d1 = batch_plane_axis( bt, axis );
             m.dv_f[ axis ][ g ] = make_udiv( unsigned( ext[ 0 ] ) );
-            m.cpp_f[ axis ][ g ] = unsigned( blocks_for( ( long long ) ext[ 0 ] * ext[ 1 ], 128 ) );
+            m.cpp_f[ axis ][ g ] = unsigned( blocks_for( ( long long ) ext[ 0 ] * ext[ d1 ], 128 ) );
+            m.warps_f[ axis ][ g ] = bt->shape[ axis ][ g ].warps;
+            m.seg_f[ axis ][ g ] = bt->shape[ axis ][ g ].seg;
         }
     }
     m.ng = int( bt->ctx.size(  ) );
@@ -290,6 +319,18 @@ static void batch_enqueue( kr_batch * bt, cudaStream_t st, T && timed )
             auto sweep = [ & ]( int kind, auto mode )
             {
                 constexpr int M = decltype( mode )::value;
+                if( M != KR_RIEMANN_LEARNED && bt->march[ axis ] )
+                {
+                    if constexpr( M != KR_RIEMANN_LEARNED )
+                    {
+                        const int nm = int( bt->cnt[ 7 - axis ] );
+                        const unsigned g = bgrid( bt, kind, 7 - axis );
+                        timed( kind, [ & ] {
+                            if( axis == 1 ) k_march_list< R, M, 1 ><<< g, 128, 0, st >>>( m, stage, nm );
+                            else            k_march_list< R, M, 2 ><<< g, 128, 0, st >>>( m, stage, nm ); } );
+                    }
+                    return;
+                }
                 const unsigned g = bgrid( bt, kind, list );
                 timed( kind, [ & ] {
                     if( axis == 0 )      k_flux_list< true, R, M, 0 ><<< g, 128, 0, st >>>( m, stage, nl );
@@ -487,7 +528,21 @@ kr_batch * kr_batch_create( kr_ctx * const * ctxs, int n )
     bt->fuse = true;
     for( int g = 0; g < n; ++ g )
         bt->fuse = bt->fuse && ctxs[ g ]->fuse_batch;
-    for( int list = 0; list < 5; ++ list )
+    long long all = 0;                       // the groups' blocks, sharing each launch
+    for( int g = 0; g < n; ++ g )
+        all += ctxs[ g ]->nblk;
+    for( int axis = 1; axis < 3; ++ axis )
+    {
+        double load = 0;
+        for( int g = 0; g < n; ++ g )
+        {
+            bt->shape[ axis ][ g ] = march_shape( ctxs[ g ]->cfg.n, axis, all,
+                                                  bt->n_sm * ( bt->precision == 1 ? march_ctas< float >(  ) : march_ctas< double >(  ) ) );
+            load += march_load( ctxs[ g ]->cfg.n, axis, ctxs[ g ]->nblk );
+        }
+        bt->march[ axis ] = march_pays( load, bt->n_sm );
+    }
+    for( int list = 0; list < KR_BATCH_LISTS; ++ list )
     {
         long long count = 0;
         for( int p = 0; p < n; ++ p )
@@ -502,14 +557,16 @@ kr_batch * kr_batch_create( kr_ctx * const * ctxs, int n )
                 tiles = tile_ctas( t );
                 planes = tile_rows( t );
             }
+            else if( list > 4 ) { tiles = bt->shape[ 7 - list ][ g ].tiles; planes = 1; }
             else
             {
                 const int axis = 2 - ( list - 1 );
                 int ext[ 3 ];
                 for( int d = 0; d < 3; ++ d )
                     ext[ d ] = ( d == axis ) ? nn[ d ] + 1 : nn[ d ] + 2;
-                tiles = blocks_for( ( long long ) ext[ 0 ] * ext[ 1 ], 128 );
-                planes = ext[ 2 ];
+                const int d1 = batch_plane_axis( bt, axis );
+                tiles = blocks_for( ( long long ) ext[ 0 ] * ext[ d1 ], 128 );
+                planes = ext[ 3 - d1 ];
             }
             bt->l_off[ list ][ p ] = int( count );
             bt->l_grp[ list ][ p ] = g;

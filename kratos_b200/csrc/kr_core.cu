@@ -1177,9 +1177,19 @@ void plm_stencil( const args_t< R > & a, int b, int axis, int step, const int * 
         ql[ BCC + axis ] = qr[ BCC + axis ] = bn;
 }
 
-// One CTA's 128 faces of a sweep: bx = CTA along the faces of one (x, y)
-// plane, by = z plane, blockIdx.z = block; dv
-// divides by the row length.
+// The second axis of the planes in which a sweep's faces are numbered for CTAs
+// and warps (x is the first, the third runs over planes): (x, y) planes, in which
+// the y sweep's CTAs share rows; in learned mode (x, z) planes for the y sweep, as
+// the march (kr_march.cuh) numbers its columns -- a warp's solver choice holds
+// for the same faces in both.  (Refined blast, y sweeps: 957 us per step in (x, y)
+// planes, 1080 in (x, z).)
+template< int MODE > __host__ __device__ constexpr int face_plane_axis( int axis )
+{
+    return axis == 1 && ( MODE == KR_RIEMANN_LEARNED || MODE == FLUX_APPLY ) ? 2 : 1;
+}
+
+// One CTA's 128 faces of a sweep, one thread per face: bx = CTA along the faces
+// of one plane, by = the plane, b = block; dv divides by the row length.
 template< bool MHD, class R, int MODE, bool XL = false > __device__ __forceinline__
 void flux_faces( const args_t< R > & a, int axis, int step, udiv_t dv, int b, unsigned bx, unsigned by,
                  bool hlle_warp = false )
@@ -1195,20 +1205,21 @@ void flux_faces( const args_t< R > & a, int axis, int step, udiv_t dv, int b, un
     int ext[ 3 ];
     for( int d = 0; d < 3; ++ d )
         ext[ d ] = d == axis ? nn[ d ] + 1 : nn[ d ] - 2 * lo;
-    total = unsigned( ext[ 0 ] * ext[ 1 ] );
+    const int d1 = face_plane_axis< MODE >( axis ), d2 = 3 - d1;
+    total = unsigned( ext[ 0 ] * ext[ d1 ] );
     if constexpr( XL )
     {   // refined MHD: one index over the whole block's faces (its blocks are
         // small, and per-plane rows of 128 faces left a fifth of the lanes idle)
         by = t / total;
         t -= by * total;
-        if( by >= unsigned( ext[ 2 ] ) )
+        if( by >= unsigned( ext[ d2 ] ) )
             return;
     }
     const unsigned q = udiv_q( t, dv );
     ii[ 0 ] = int( t - q * unsigned( ext[ 0 ] ) );
-    ii[ 1 ] = int( q );
-    ii[ 2 ] = int( by );
-    t_lin = ( long long ) t + ( long long ) total * by;
+    ii[ d1 ] = int( q );
+    ii[ d2 ] = int( by );
+    t_lin = ii[ 0 ] + ( long long ) ext[ 0 ] * ( ii[ 1 ] + ( long long ) ext[ 1 ] * ii[ 2 ] );
     for( int d = 0; d < 3; ++ d )
         if( d != axis )
         {
@@ -1221,7 +1232,7 @@ void flux_faces( const args_t< R > & a, int axis, int step, udiv_t dv, int b, un
     if( ! valid && ! learned )
         return;
     // learned mode: the warp's place in the sweep's chunk order (chunks of 128
-    // faces, z plane outer, 4 warps each)
+    // faces, planes outer, 4 warps each)
     const unsigned wid = ( by * ( ( total + 127u ) >> 7 ) + bx ) * 4u + ( threadIdx.x >> 5 );
     const int st = axis == 0 ? 1 : ( axis == 1 ? a.sw1 : a.sw2 );
     R ql[ 8 ], qr[ 8 ];
@@ -1275,6 +1286,8 @@ k_flux_eval( const args_t< R > a, int step, udiv_t dv, unsigned cpp, unsigned nz
     for( unsigned ch = blockIdx.x; ch < cpp * nz; ch += gridDim.x )
         flux_faces< MHD, R, KR_RIEMANN_LEARNED >( a, axis, step, dv, blockIdx.z, ch % cpp, ch / cpp );
 }
+
+#include "kr_march.cuh"
 
 ////////////////////////////////////////////////////////////
 // Edge EMF (mhd/integrator/integrator.h:189-327 calc_field): face EMF average
@@ -2159,6 +2172,7 @@ struct kr_ctx
     kr_cfg cfg;
     std::string err;
     int nblk = 0, nw = 0, nws = 0, nf = 0;   // nw: host words / cell; nws: stored W words
+    long long nblk_mesh = 0;                 // blocks of the whole mesh (all ranks)
     long long nc = 0, ngw = 0, nbf = 0, nfb = 0;
     size_t rsize = 8;
     cudaStream_t stream = nullptr;
@@ -2307,31 +2321,47 @@ static long long phys_sites( const kr_ctx * c )
 template< bool MHD, class R, int MODE, int axis >
 static void launch_flux_axis( kr_ctx * c, cudaStream_t st, const args_t< R > & a, int stage )
 {
-    // one thread per face of the sweep, the MHD transverse ghost lines included
+    // every face of the sweep, the MHD transverse ghost lines included
     const int * n = c->cfg.n;
-    int ext[ 3 ];
+    long long ext[ 3 ];
     for( int d = 0; d < 3; ++ d )
         ext[ d ] = ( d == axis ) ? n[ d ] + 1 : n[ d ] + ( MHD ? 2 : 0 );
+    const int d1 = face_plane_axis< MODE >( axis ), d2 = 3 - d1;
+    const unsigned cpp = blocks_for( ext[ 0 ] * ext[ d1 ], 128 );
+    const udiv_t dv = make_udiv( unsigned( ext[ 0 ] ) );
     if constexpr( MODE == KR_RIEMANN_LEARNED && MHD )
     {
-        const unsigned cpp = blocks_for( ( long long ) ext[ 0 ] * ext[ 1 ], 128 );
         const unsigned ge = unsigned( std::max< long long >( 1, std::min< long long >(
-            ( long long ) cpp * ext[ 2 ], ( 2LL * c->n_sm * flux_min_ctas< R, KR_RIEMANN_LEARNED >(  ) ) / c->nblk ) ) );
-        k_flux_eval< MHD, R, axis ><<< dim3( ge, 1, c->nblk ), 128, 0, st >>>(
-            a, stage, make_udiv( unsigned( ext[ 0 ] ) ), cpp, unsigned( ext[ 2 ] ) );
+            cpp * ext[ d2 ], ( 2LL * c->n_sm * flux_min_ctas< R, KR_RIEMANN_LEARNED >(  ) ) / c->nblk ) ) );
+        k_flux_eval< MHD, R, axis ><<< dim3( ge, 1, c->nblk ), 128, 0, st >>>( a, stage, dv, cpp, unsigned( ext[ d2 ] ) );
     }
     // sweeps without the network: each warp of faces runs the solver chosen
     // for it (exits at once on the network's sweep)
     constexpr int M = ( MODE == KR_RIEMANN_LEARNED && MHD ) ? FLUX_APPLY : MODE;
-    const dim3 grid( blocks_for( ( long long ) ext[ 0 ] * ext[ 1 ], 128 ), ext[ 2 ], c->nblk );
-    if constexpr( MHD && ( MODE == KR_RIEMANN_DEFAULT || MODE == KR_RIEMANN_HLLE ) )
-        if( c->smr )
-        {   // one flat index over each block's faces (flux_faces, XL)
-            const dim3 flat( blocks_for( ( long long ) ext[ 0 ] * ext[ 1 ] * ext[ 2 ], 128 ), 1, c->nblk );
-            k_flux< MHD, R, M, true, axis ><<< flat, 128, 0, st >>>( a, stage, make_udiv( unsigned( ext[ 0 ] ) ) );
+    constexpr bool refined = MHD && ( MODE == KR_RIEMANN_DEFAULT || MODE == KR_RIEMANN_HLLE );
+    if constexpr( MHD && axis != 0 && M != FLUX_SAMPLE )
+        if( ! ( axis == 1 && c->smr ) && march_pays( march_load( n, axis, c->nblk_mesh ), c->n_sm ) )
+        {   // (refined meshes: z only; on the blast's 16^3 blocks the y march
+            // took 1038 us per step against k_flux's 957, the z march 822 against 939)
+            const march_t m = march_shape( n, axis, c->nblk, c->n_sm * march_ctas< R >(  ) );
+            const dim3 grid( m.tiles, 1, c->nblk );
+            if constexpr( refined && axis == 2 )
+                if( c->smr )
+                {
+                    k_march< R, M, true, axis ><<< grid, 128, 0, st >>>( a, stage, dv, m.warps, m.seg );
+                    return;
+                }
+            k_march< R, M, false, axis ><<< grid, 128, 0, st >>>( a, stage, dv, m.warps, m.seg );
             return;
         }
-    k_flux< MHD, R, M, false, axis ><<< grid, 128, 0, st >>>( a, stage, make_udiv( unsigned( ext[ 0 ] ) ) );
+    if constexpr( refined )
+        if( c->smr )
+        {   // one flat index over each block's faces (flux_faces, XL)
+            const dim3 flat( blocks_for( ext[ 0 ] * ext[ 1 ] * ext[ 2 ], 128 ), 1, c->nblk );
+            k_flux< MHD, R, M, true, axis ><<< flat, 128, 0, st >>>( a, stage, dv );
+            return;
+        }
+    k_flux< MHD, R, M, false, axis ><<< dim3( cpp, unsigned( ext[ d2 ] ), c->nblk ), 128, 0, st >>>( a, stage, dv );
 }
 
 template< bool MHD, class R, int MODE >
@@ -2931,6 +2961,7 @@ static kr_ctx * create_ctx( const kr_cfg * cfg, int n_regions, const kr_region *
         halo_plan( * cfg, owner, local, halo_all, c->hsend, c->hrecv );
     }
     c->nblk = int( c->gid_h.size(  ) );
+    c->nblk_mesh = smr ? c->nblk : ( long long ) cfg->nb[ 0 ] * cfg->nb[ 1 ] * cfg->nb[ 2 ];
     if( c->hsend.items.size(  ) > 65535 || c->hrecv.items.size(  ) > 65535 )
     {   // one grid row per item
         g_create_error = "kr_ctx_create: more than 65535 halo items on one rank";
@@ -3016,7 +3047,8 @@ static kr_ctx * create_ctx( const kr_cfg * cfg, int n_regions, const kr_region *
             long long ext[ 3 ];
             for( int d = 0; d < 3; ++ d )
                 ext[ d ] = d == ax ? n[ d ] + 1 : n[ d ] + 2;
-            c->sel_wcap = std::max( c->sel_wcap, blocks_for( ext[ 0 ] * ext[ 1 ], 128 ) * ext[ 2 ] * 4 );
+            const int d1 = face_plane_axis< KR_RIEMANN_LEARNED >( ax );
+            c->sel_wcap = std::max( c->sel_wcap, blocks_for( ext[ 0 ] * ext[ d1 ], 128 ) * ext[ 3 - d1 ] * 4 );
         }
         const size_t bytes = size_t( 3 ) * nb * c->sel_wcap * sizeof( unsigned );
         ok = ck( c, cudaMalloc( & c->sel_dec, bytes ), "malloc selector choices" )

@@ -125,9 +125,9 @@ void plm_face_fast2( float2 q_ll, float2 q_l, float2 q_r, float2 q_rr, float2 & 
     const float2 sl = __fadd2_rn( dql, dqc ), sr = __fadd2_rn( dqc, dqr );
     const float2 il = make_float2( rcp( sl.x ), rcp( sl.y ) ), ir = make_float2( rcp( sr.x ), rcp( sr.y ) );
     const float2 tl = __fmul2_rn( dqc, il );
-    const float2 tr = __fmul2_rn( __fmul2_rn( dqc, ir ), m1 );
+    const float2 tr = __fmul2_rn( __fmul2_rn( dqr, ir ), m1 );
     const float2 cl = __ffma2_rn( dql, tl, q_l );        // q_l + dql ( dqc / ( dql + dqc ) )
-    const float2 cr = __ffma2_rn( dqr, tr, q_r );        // q_r - dqr ( dqc / ( dqc + dqr ) )
+    const float2 cr = __ffma2_rn( dqc, tr, q_r );        // q_r - dqc ( dqr / ( dqc + dqr ) )
     ql = make_float2( lx ? cl.x : q_l.x, ly ? cl.y : q_l.y );
     qr = make_float2( rx ? cr.x : q_r.x, ry ? cr.y : q_r.y );
 }

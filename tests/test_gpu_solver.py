@@ -74,3 +74,30 @@ def test_one_step_from_random_states(nb, n, flow, precision):
     own = np.s_[:, 2:n[2] + 2, 2:n[1] + 2, 2:n[0] + 2]
     assert np.abs(b[own] - bo[own]).sum() <= tol * max(np.abs(bo[own]).sum(), np.abs(u0[..., 0]).sum())
     d.close()
+
+
+@pytest.mark.parametrize("precision", [2, 1])
+@pytest.mark.parametrize("kw", [{}, {"integrator": 1}])
+@pytest.mark.parametrize("nb,n", [((1, 1, 1), (130, 131, 70)), ((10, 10, 10), (9, 12, 17)), ((2, 1, 2), (300, 9, 101))])
+def test_marching_sweeps(nb, n, kw, precision):
+    """Meshes large enough for the y and z sweeps to march (columns that end in
+    partial warps, one and many blocks, short and long runs of faces)."""
+    from kratos_b200 import Dynamics
+    from oracle.kr_oracle import OracleMesh
+    u0, b0 = _state(nb, n, "subsonic", 11)
+    o = OracleMesh(True, nb, n, GAMMA, **kw)
+    o.set_state(u0, b0)
+    o.step(2)
+    uo, bo = o.get_state()
+    d = Dynamics(True, nb, n, gamma=GAMMA, precision=precision, **kw)
+    d.set_state(u0, b0)
+    d.step(2)
+    u, b = d.get_state()
+    assert d.status() == 0
+    tol = 1e-11 if precision == 2 else 2e-5
+    for k in range(5):
+        scale = np.abs(uo[..., 2:5]).max(-1).sum() if k >= 2 else np.abs(uo[..., k]).sum()
+        assert np.abs(u[..., k] - uo[..., k]).sum() <= tol * scale, "field %d" % k
+    own = np.s_[:, 2:n[2] + 2, 2:n[1] + 2, 2:n[0] + 2]
+    assert np.abs(b[own] - bo[own]).sum() <= tol * np.abs(bo[own]).sum()
+    d.close()
