@@ -71,25 +71,13 @@ struct multi_scal_t
 __global__ void k_step_begin_multi( const __grid_constant__ multi_scal_t m )
 {
     for( int g = 0; g < m.n; ++ g )
-        for( int k = 0; k < m.ns[ g ]; ++ k )
-            m.s[ g ][ k ].dt_bits = __double_as_longlong( m.s[ g ][ k ].dt_bound );
+        step_begin( m.s[ g ], m.ns[ g ] );
 }
 
 __global__ void k_step_end_multi( const __grid_constant__ multi_scal_t m, double dt_expand )
 {
     for( int g = 0; g < m.n; ++ g )
-        for( int k = 0; k < m.ns[ g ]; ++ k )
-        {
-            scal_t & r = m.s[ g ][ k ];
-            const double dt = __longlong_as_double( r.dt_bits );
-            if( ! ( dt > 0 ) || ! isfinite( dt ) )
-                m.s[ g ][ 0 ].status |= 1;
-            r.dt_last  = dt;
-            r.t       += dt;
-            r.dt_bound = dt * dt_expand;
-            r.n_steps += 1;
-            r.sel_force = 0;
-        }
+        step_end( m.s[ g ], dt_expand, m.ns[ g ] );
 }
 
 // item: x group, y block, z plane, w tile
@@ -304,7 +292,7 @@ static void batch_enqueue( kr_batch * bt, cudaStream_t st, T && timed )
 {
     const multi_t< R > m = make_multi< R >( bt );
     const multi_scal_t ms = make_multi_scal( bt );
-    k_step_begin_multi<<< 1, 1, 0, st >>>( ms );
+    k_step_begin_multi<<< 1, 256, 0, st >>>( ms );
     const bool learned = bt->riemann == KR_RIEMANN_LEARNED;
     for( int stage = 0; stage < 2; ++ stage )
     {
@@ -358,7 +346,7 @@ static void batch_enqueue( kr_batch * bt, cudaStream_t st, T && timed )
         timed( BK_UPD1, [ & ] { k_update_list< true, R, 1 ><<< bgrid( bt, BK_UPD1, 0 ), 256, 0, st >>>( m, stage, int( bt->cnt[ 0 ] ) ); } );
         timed( BK_UPD2, [ & ] { k_update_list< true, R, 2 ><<< bgrid( bt, BK_UPD2, 4 ), 256, 0, st >>>( m, stage, ne ); } );
     }
-    k_step_end_multi<<< 1, 1, 0, st >>>( ms, bt->ctx[ 0 ]->cfg.dt_expand );
+    k_step_end_multi<<< 1, 256, 0, st >>>( ms, bt->ctx[ 0 ]->cfg.dt_expand );
 }
 
 static void batch_drop_graph( kr_batch * bt )
