@@ -3,7 +3,7 @@
 //
 // Every kernel kind of the step runs as ONE persistent launch whose CTAs walk
 // a work list: one item per CTA tile that the per-group launches would run
-// (group, block, plane or row of planes, tile along it), bigger blocks first.  A CTA
+// (group, block, plane of a sweep, tile), bigger blocks first.  A CTA
 // takes items blockIdx.x, blockIdx.x + gridDim.x, ... and runs the same
 // per-site code on the item's group arguments (read from the kernel's
 // parameter space by the item's group index), so a batched step gives the
@@ -35,8 +35,8 @@ struct multi_t
     // the work lists [cells | flux z | flux y | flux x | lattice sites | the z and
     // y marches]: per list,
     // the first item of each group in list order (l_off[.][ng] = the count),
-    // that group, and its tiles per plane (cells, lattice: per row of planes)
-    // and planes per block
+    // that group, and its tiles per plane and planes per block (cells, lattice and
+    // the marches: one plane)
     int ng;
     int l_off[ KR_BATCH_LISTS ][ KR_BATCH_MAX + 1 ];
     int l_grp[ KR_BATCH_LISTS ][ KR_BATCH_MAX ];
@@ -88,7 +88,7 @@ k_c2p_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
         const int4 t = batch_item( m, 0, it );
-        c2p_cells< MHD, R, DT >( m.a[ t.x ], step, m.cells[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
+        c2p_cells< MHD, R, DT >( m.a[ t.x ], step, m.cells[ t.x ], t.y, unsigned( t.w ) * 256u + threadIdx.x );
         if( DT )
             __syncthreads(  );            // the CTA reduction's shared words are reused
     }
@@ -149,7 +149,7 @@ k_emf_list( const __grid_constant__ multi_t< R > m, int n_items )
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
         const int4 t = batch_item( m, 4, it );
-        emf_site< R >( m.a[ t.x ], m.lattice[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
+        emf_site< R >( m.a[ t.x ], m.lattice[ t.x ], t.y, unsigned( t.w ) * 256u + threadIdx.x );
     }
 }
 
@@ -160,7 +160,7 @@ k_update_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
     for( int it = blockIdx.x; it < n_items; it += gridDim.x )
     {
         const int4 t = batch_item( m, PART == 1 ? 0 : 4, it );
-        update_site< MHD, R, false, PART >( m.a[ t.x ], step, PART == 1 ? m.cells[ t.x ] : m.lattice[ t.x ], t.y, t.z, unsigned( t.w ) * 256u + threadIdx.x );
+        update_site< MHD, R, false, PART >( m.a[ t.x ], step, PART == 1 ? m.cells[ t.x ] : m.lattice[ t.x ], t.y, unsigned( t.w ) * 256u + threadIdx.x );
     }
 }
 
@@ -174,7 +174,7 @@ k_update_c2p_list( const __grid_constant__ multi_t< R > m, int n_items )
     {
         const int4 t = batch_item( m, 0, it );
         int i[ 3 ];
-        if( tile_site( m.cells[ t.x ], t.z, unsigned( t.w ) * 256u + threadIdx.x, i ) )
+        if( tile_site( m.cells[ t.x ], unsigned( t.w ) * 256u + threadIdx.x, i ) )
             update_c2p_cell< R >( m.a[ t.x ], t.y, i[ 0 ], i[ 1 ], i[ 2 ] );
     }
 }
@@ -543,7 +543,7 @@ kr_batch * kr_batch_create( kr_ctx * const * ctxs, int n )
                 const int e = list == 4;
                 const tile_t t = make_tile( nn[ 0 ] + e, nn[ 1 ] + e, nn[ 2 ] + e );
                 tiles = tile_ctas( t );
-                planes = tile_rows( t );
+                planes = 1;
             }
             else if( list > 4 ) { tiles = bt->shape[ 7 - list ][ g ].tiles; planes = 1; }
             else

@@ -18,6 +18,7 @@
 // stage 0's two updates and stage 1's c2p are one launch (k_update_c2p).
 #include "../../include/kratos_b200.h"
 #include "kr_fast.cuh"
+#include "kr_index.h"
 #include "kr_mlp.cuh"
 #include "problems.h"
 #include "smr_tree.h"
@@ -195,54 +196,6 @@ long long ifx( const args_t< R > & a, int b, int c, int nf, int i0, int i1, int 
     return ( long long )( b * nf + c ) * a.nfb + ( i0 + 1 ) + a.sf1 * ( i1 + 1 ) + a.sf2 * ( i2 + 1 );
 }
 
-// Quotient of a non-negative n by a fixed d >= 2 with one multiply-high:
-// q = umulhi( n, ceil( 2^32 / d ) ), exact while n * d < 2^32 (the rounding
-// error of the multiplier, below d, times n stays under 2^32).
-struct udiv_t { unsigned d, m; };
-static inline udiv_t make_udiv( unsigned d )
-{
-    return { d, unsigned( ( ( 1ull << 32 ) + d - 1 ) / d ) };
-}
-__device__ __forceinline__ unsigned udiv_q( unsigned n, const udiv_t & v ) { return __umulhi( n, v.m ); }
-
-__device__ __forceinline__ unsigned udiv_q1( unsigned n, const udiv_t & v )   // d >= 1
-{
-    return v.d == 1 ? n : udiv_q( n, v );
-}
-
-// The sites of a block (e0 x e1 x e2, x fastest) over CTAs of 256 threads: a
-// row of CTAs walks `g` planes as one index, so small planes share CTAs (the
-// 17 x 17 edge sites of a 16^3 block's plane filled 56% of two CTAs, its 17
-// planes fill 96% of 20).  g: all planes, or as many as keep the quotients exact.
-struct tile_t
-{
-    int e0, e1, e2, g;
-    udiv_t d0, d01;
-};
-static inline tile_t make_tile( int e0, int e1, int e2 )
-{
-    const long long p = ( long long ) e0 * e1;
-    const long long most = std::max( 1LL, std::min< long long >( e2, ( ( 1LL << 32 ) - 1 ) / ( p * p ) ) );
-    const long long rows = ( e2 + most - 1 ) / most;
-    return { e0, e1, e2, int( ( e2 + rows - 1 ) / rows ), make_udiv( unsigned( e0 ) ), make_udiv( unsigned( p ) ) };
-}
-static inline unsigned tile_ctas( const tile_t & t )
-{
-    return unsigned( ( ( long long ) t.e0 * t.e1 * t.g + 255 ) / 256 );
-}
-static inline unsigned tile_rows( const tile_t & t ) { return unsigned( ( t.e2 + t.g - 1 ) / t.g ); }
-
-// Site s of row `row`; false past the block's last site.
-__device__ __forceinline__ bool tile_site( const tile_t & t, int row, unsigned s, int * i )
-{
-    const unsigned p = t.g == 1 ? 0u : udiv_q( s, t.d01 ), r = s - p * t.d01.d;
-    const unsigned q = udiv_q( r, t.d0 );
-    i[ 0 ] = int( r - q * t.d0.d );
-    i[ 1 ] = int( q );
-    i[ 2 ] = row * t.g + int( p );
-    return i[ 1 ] < t.e1 && int( p ) < t.g && i[ 2 ] < t.e2;
-}
-
 __device__ __forceinline__ double warp_min( double v )
 {
     for( int o = 16; o > 0; o >>= 1 )
@@ -363,14 +316,14 @@ void c2p_point( const args_t< R > & a, R * W, double * U, int b, int i0, int i1,
 
 // DT: stage 0's launch, which also reduces the CFL dt; stage 1's launch has none
 // of that code (fewer registers).
-// One CTA's cells: block b, site c of row `row` of its cells (every thread of
-// the CTA calls it: the dt reduction is CTA-wide).
+// One CTA's cells: block b, site c of its cells (every thread of the CTA calls
+// it: the dt reduction is CTA-wide).
 template< bool MHD, class R, bool DT > __device__ __forceinline__
-void c2p_cells( const args_t< R > & a, int step, const tile_t & tl, int b, int row, unsigned c )
+void c2p_cells( const args_t< R > & a, int step, const tile_t & tl, int b, unsigned c )
 {
     double dt = FLT_MAX;
     int ic[ 3 ];
-    if( tile_site( tl, row, c, ic ) )
+    if( tile_site( tl, c, ic ) )
     {
         const int i0 = ic[ 0 ], i1 = ic[ 1 ], i2 = ic[ 2 ];
         double * U = a.u[ step ];
@@ -448,8 +401,8 @@ void c2p_cells( const args_t< R > & a, int step, const tile_t & tl, int b, int r
 template< bool MHD, class R, bool DT >
 __global__ void __launch_bounds__( 256, ( MHD && DT ) ? 3 : 4 ) k_c2p( const args_t< R > a, int step, tile_t tl )
 {
-    // grid: x, y over the block's cells (tile_t), z over blocks
-    c2p_cells< MHD, R, DT >( a, step, tl, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
+    // grid: x over the block's cells (tile_t), z over blocks
+    c2p_cells< MHD, R, DT >( a, step, tl, blockIdx.z, blockIdx.x * blockDim.x + threadIdx.x );
 }
 
 ////////////////////////////////////////////////////////////
@@ -1310,12 +1263,12 @@ R face_emf( const args_t< R > & a, int b, int fa, int ax, const int * i )
     return a.f[ fa ][ ifx( a, b, slot, 7, i[ 0 ], i[ 1 ], i[ 2 ] ) ];
 }
 
-// Edge site t of row `row` of block b.
+// Edge site t of block b.
 template< class R > __device__ __forceinline__
-void emf_site( const args_t< R > & a, const tile_t & tl, int b, int row, unsigned t )
+void emf_site( const args_t< R > & a, const tile_t & tl, int b, unsigned t )
 {
     int i[ 3 ];
-    if( ! tile_site( tl, row, t, i ) )
+    if( ! tile_site( tl, t, i ) )
         return;
     const int nn[ 3 ] = { a.n0, a.n1, a.n2 };
     const R w_e = R( 0.25f );
@@ -1389,8 +1342,8 @@ void emf_site( const args_t< R > & a, const tile_t & tl, int b, int row, unsigne
 template< class R >
 __global__ void __launch_bounds__( 256 ) k_emf( const args_t< R > a, tile_t tl )
 {
-    // grid: x, y over the block's edge sites (tile_t), z over blocks
-    emf_site< R >( a, tl, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
+    // grid: x over the block's edge sites (tile_t), z over blocks
+    emf_site< R >( a, tl, blockIdx.z, blockIdx.x * blockDim.x + threadIdx.x );
 }
 
 ////////////////////////////////////////////////////////////
@@ -1558,14 +1511,14 @@ double ct_face( const args_t< R > & a, const geo_t & g, int b, int c, const int 
 }
 
 // PART 1: the conserved update of the cells; 2 (MHD): the CT update of the faces
-// (two launches, each with fewer registers).  Site t of row `row` of block b: a
-// cell, or a lattice site (its three lower faces).
+// (two launches, each with fewer registers).  Site t of block b: a cell, or a lattice
+// site (its three lower faces).
 template< bool MHD, class R, bool SMR, int PART > __device__ __forceinline__
-void update_site( const args_t< R > & a, int step, const tile_t & tl, int b, int row, unsigned t )
+void update_site( const args_t< R > & a, int step, const tile_t & tl, int b, unsigned t )
 {
     constexpr int NF = MHD ? 7 : 5;
     int i[ 3 ];
-    if( ! tile_site( tl, row, t, i ) )
+    if( ! tile_site( tl, t, i ) )
         return;
     const int nn[ 3 ] = { a.n0, a.n1, a.n2 };
     // Heun: U* = U + dt L(U), U' = (U + U*) / 2 + dt / 2 L(U*); VL2:
@@ -1706,8 +1659,8 @@ void update_site( const args_t< R > & a, int step, const tile_t & tl, int b, int
 template< bool MHD, class R, bool SMR, int PART >
 __global__ void __launch_bounds__( 256, ( SMR && sizeof( R ) == 4 ) ? 4 : ( PART == 2 ? 6 : 4 ) ) k_update( const args_t< R > a, int step, tile_t tl )
 {
-    // grid: x, y over the block's cells or lattice sites (tile_t), z over blocks
-    update_site< MHD, R, SMR, PART >( a, step, tl, blockIdx.z, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x );
+    // grid: x over the block's cells or lattice sites (tile_t), z over blocks
+    update_site< MHD, R, SMR, PART >( a, step, tl, blockIdx.z, blockIdx.x * blockDim.x + threadIdx.x );
 }
 
 ////////////////////////////////////////////////////////////
@@ -1763,9 +1716,9 @@ void update_c2p_cell( const args_t< R > & a, int b, int i0, int i1, int i2 )
 template< class R >
 __global__ void __launch_bounds__( 256, 4 ) k_update_c2p( const args_t< R > a, tile_t tl )
 {
-    // grid: x, y over the block's cells (tile_t), z over blocks
+    // grid: x over the block's cells (tile_t), z over blocks
     int i[ 3 ];
-    if( tile_site( tl, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x, i ) )
+    if( tile_site( tl, blockIdx.x * blockDim.x + threadIdx.x, i ) )
         update_c2p_cell< R >( a, blockIdx.z, i[ 0 ], i[ 1 ], i[ 2 ] );
 }
 
@@ -2386,7 +2339,7 @@ static void launch_flux_mode( kr_ctx * c, cudaStream_t st, const args_t< R > & a
     else                                          launch_flux< MHD, R, KR_RIEMANN_DEFAULT >( c, st, a, axis, stage );
 }
 
-static dim3 tile_grid( const tile_t & t, unsigned nblk ) { return dim3( tile_ctas( t ), tile_rows( t ), nblk ); }
+static dim3 tile_grid( const tile_t & t, unsigned nblk ) { return dim3( tile_ctas( t ), 1, nblk ); }
 
 // One stage is front (cons -> prim, CFL dt at stage 0, pack of the halo other
 // ranks read), exchange (NCCL send / receive by peer; at stage 0 the dt
