@@ -560,17 +560,9 @@ kr_batch * kr_batch_create( kr_ctx * const * ctxs, int n )
             bt->l_grp[ list ][ p ] = g;
             bt->l_tiles[ list ][ p ] = make_udiv( unsigned( tiles ) );
             bt->l_planes[ list ][ p ] = make_udiv( unsigned( planes ) );
-            const long long items = tiles * planes * ctxs[ g ]->nblk;
-            // the multiply-high quotients are exact while item * divisor < 2^32
-            if( items * std::max( tiles, planes ) >= ( 1LL << 32 ) )
-            {
-                g_create_error = "kr_batch_create: a box group's work list is too long for 32-bit item decoding";
-                delete bt;
-                return nullptr;
-            }
-            count += items;
+            count += tiles * planes * ctxs[ g ]->nblk;
         }
-        if( count >= ( 1LL << 31 ) )
+        if( count >= ( 1LL << 31 ) )         // items are ints, their quotients exact below that
         {
             g_create_error = "kr_batch_create: a work list of more than 2^31 items";
             delete bt;

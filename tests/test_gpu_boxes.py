@@ -167,3 +167,17 @@ def test_batch_autotune_caches_and_keeps_state(tmp_path):
     bb.step(2)
     assert bb.status() == 0
     bb.close()
+
+
+def test_batch_of_long_boxes():
+    """Boxes whose sites are one long list of tiles (25 x 33 x 6301 lattice sites:
+    20,306 tiles, times 13 boxes times 20,306 above 2^32) join a batch."""
+    import ctypes
+
+    from kratos_b200 import Dynamics
+    from kratos_b200 import _lib as L
+    d = Dynamics(True, (13, 1, 1), (24, 32, 6300), gamma=5 / 3, precision=1, flags=L.KR_FLAG_BOXES)
+    bt = L.lib().kr_batch_create((ctypes.c_void_p * 1)(d._h), 1)
+    assert bt, L.lib().kr_batch_last_error(None).decode()
+    L.lib().kr_batch_destroy(bt)
+    d.close()

@@ -14,8 +14,29 @@ MAIN = r"""
 #include <cstdlib>
 #include "kr_index.h"
 using namespace kr;
+// every divisor's quotients at, just below and just above multiples of it, up to 2^31
+static long long quotients(  )
+{
+    long long bad = 0;
+    for( unsigned k = 1; k < 40000; ++ k )
+    {
+        const unsigned d = k < 20000 ? k : unsigned( 1 + k * 53681ull % 2147483000ull );
+        const udiv_t v = make_udiv( d );
+        const unsigned top = 0x7fffffffu / d;
+        for( unsigned j = 0; j < 400; ++ j )
+        {
+            const unsigned q = j < 200 ? std::min( j, top ) : top - std::min( j - 200, top );
+            for( long long n = ( long long ) q * d - 1; n <= ( long long ) q * d + 1; ++ n )
+                if( n >= 0 && n < ( 1LL << 31 ) )
+                    bad += udiv_q1( unsigned( n ), v ) != unsigned( n ) / d;
+        }
+    }
+    return bad;
+}
 int main( int argc, char ** argv )
 {
+    if( argc == 1 )
+        return std::printf( "%lld\n", quotients(  ) ) < 0;
     const int n[ 3 ] = { atoi( argv[ 1 ] ), atoi( argv[ 2 ] ), atoi( argv[ 3 ] ) };
     long long rows = 0, sites = 0;
     const udiv_t dv = make_udiv( unsigned( n[ 0 ] + 2 ) );
@@ -52,3 +73,8 @@ def exe(tmp_path_factory):
 def test_every_site_and_row(exe, n):
     out = subprocess.run([exe] + [str(k) for k in n], capture_output=True, text=True, check=True).stdout.split()
     assert out == ["0", "0"], "wrong rows of the faces' planes, wrong sites of the tiles: %s" % out
+
+
+def test_quotients_below_2_to_31(exe):
+    out = subprocess.run([exe], capture_output=True, text=True, check=True).stdout.split()
+    assert out == ["0"], "wrong quotients: %s" % out
