@@ -214,10 +214,20 @@ void hllc_fast( R * flx, const R * wl, const R * wr, const eos_c< R > & e )
 // state is degenerate (f_tiny below) the reference keeps the outer transverse
 // field, whose jump the contact speed does not satisfy: the field flux then takes
 // the difference B_t (v_n - S_M).
-// Flux sweeps z / y / x of the 256^3 mesh in 64 blocks of 64^3, ms per launch,
-// with the reciprocals above: FP64 1.62 / 1.50 / 1.41 -> 0.67 / 0.65 / 0.58, FP32
-// 0.48 / 0.45 / 0.37 -> 0.35 / 0.33 / 0.31.  FP32 states against FP64 after 6 to
-// 12 steps of a smooth flow: 0.4 to 0.5 of the two-sided form's distance.
+// FP32 forms the star states as the outer state plus a difference that is itself
+// made of the states' differences: S_M - v_n = ( m' dv_n - dp_T ) / dm (m' the other
+// side's rho ( S - v_n )), rho* - rho, E* - E, B_t* - B_t and v_t** - v_t* all carry
+// it as a factor.  Formed directly, S_M and the star states each bring the rounding
+// of large sums into a flux whose outer wave may be nearly at rest: one step of
+// Mach 5 turbulence at beta 0.1 (96^3) moved the face fields 2.5e-8 to 2.9e-8 (L1)
+// from FP64, the outer flux plus jumps of directly formed states 1.3e-8 to 1.4e-8,
+// this 1.0e-8 to 1.3e-8.  Over turbulence, vortices, boxes and VL2, 5 to 12 steps,
+// every field's 2-norm error is 0.3 to 0.95 of that two-sided form's.
+// Flux sweeps z / y / x of the 256^3 mesh in 64 blocks of 64^3, ms per launch, one
+// thread per face, two-sided -> one-sided with the reciprocals above: FP64 1.62 /
+// 1.50 / 1.41 -> 0.67 / 0.65 / 0.58, FP32 0.48 / 0.45 / 0.37 -> 0.35 / 0.33 / 0.31
+// (direct and difference forms alike: 600 / 643 / 704 and 611 / 643 / 708 us per step
+// with the march).
 
 template< class R > struct lr_t;
 template<> struct lr_t< float >  { typedef float2 type; };
@@ -284,91 +294,122 @@ void hlld_tail( R * flx, const hll_prefix< R > & h, const eos_c< R > & e )
     typedef lr< R > P;
     const R b_x = h.b_x, bx_2 = h.bx_2;
     const R f_tiny = R( 1.00e-4f );
-    const P nb2 = mk2( -bx_2, -bx_2 ), bx = mk2( b_x, b_x );
+    constexpr bool F32 = sizeof( R ) == 4;
+    const P nb2 = mk2( -bx_2, -bx_2 ), nbx = mk2( -b_x, -b_x );
     const P pt = add2( h.pre, h.pm );
     const P s2 = mk2( h.spd_m2, h.spd_p2 );
     const P sd = sub2( s2, h.vn );
     const P m = mul2( h.rho, sd );                              // rho ( S - v_n )
     const P u_m = mul2( h.rho, h.vn );
-    const R spd0 = ( sd.y * u_m.y - pt.y - sd.x * u_m.x + pt.x ) * rcp( m.y - m.x );
-    const P s0 = mk2( spd0, spd0 );
-    const P sdm = sub2( s2, s0 ), dv = sub2( h.vn, s0 );
-    const R ptot_s = pt.x - m.x * dv.x;
-    P ism;
-    if constexpr( sizeof( R ) == 4 )
+    P s0, w, sdm, ism;                                          // S_M, S_M - v_n, S - S_M
+    if constexpr( F32 )
+    {   // from the states' differences (above)
+        const R dv = h.vn.y - h.vn.x, dp = pt.y - pt.x, i = rcp( m.y - m.x );
+        w = mk2( ( m.y * dv - dp ) * i, ( m.x * dv - dp ) * i );
+        s0 = add2( h.vn, w );
+        sdm = sub2( sd, w );
         ism = rcp2( sdm );
+    }
     else
-    {   // one reciprocal for both sides
-        const R i = rcp( sdm.x * sdm.y );
+    {
+        const R sc = ( sd.y * u_m.y - pt.y - sd.x * u_m.x + pt.x ) * rcp( m.y - m.x );
+        s0 = mk2( sc, sc );
+        w = sub2( s0, h.vn );
+        sdm = sub2( s2, s0 );
+        const R i = rcp( sdm.x * sdm.y );                       // one reciprocal for both sides
         ism = mk2( sdm.y * i, sdm.x * i );
     }
+    const R ptot_s = pt.x + m.x * w.x;
     const P rhos = mul2( m, ism );
     const P rs = rsq2( rhos );                                  // 1 / sqrt( rho* )
     const P sq = mul2( rhos, rs );
     const P denom = mad2( m, sdm, nb2 );
     const P id = rcp2( denom );
-    P tv = mul2( mul2( bx, dv ), id );
-    P tb = mul2( mad2( m, sd, nb2 ), id );
-    const R flat = f_tiny * ptot_s;
+    P tv = mul2( mul2( nbx, w ), id );                          // v_t* = v_t + B_t tv
+    P tb;                                                       // B_t* = B_t tb (FP32: B_t + B_t tb)
+    if constexpr( F32 ) tb = mul2( mul2( m, w ), id );
+    else                tb = mul2( mad2( m, sd, nb2 ), id );
+    const R flat = f_tiny * ptot_s, keep = R( F32 ? 0 : 1 );
     const bool flat_l = uabs( denom.x ) < flat, flat_r = uabs( denom.y ) < flat;
     tv = mk2( flat_l ? R( 0 ) : tv.x, flat_r ? R( 0 ) : tv.y );
-    tb = mk2( flat_l ? R( 1 ) : tb.x, flat_r ? R( 1 ) : tb.y );
+    tb = mk2( flat_l ? keep : tb.x, flat_r ? keep : tb.y );
     const P vs1 = mad2( h.bt1, tv, h.vt1 ), vs2 = mad2( h.bt2, tv, h.vt2 );
-    const P bs1 = mul2( h.bt1, tb ), bs2 = mul2( h.bt2, tb );
-    const R spd_m1 = spd0 - uabs( b_x ) * rs.x, spd_p1 = spd0 + uabs( b_x ) * rs.y;
+    P bs1, bs2;
+    if constexpr( F32 ) { bs1 = mad2( h.bt1, tb, h.bt1 ); bs2 = mad2( h.bt2, tb, h.bt2 ); }
+    else                { bs1 = mul2( h.bt1, tb ); bs2 = mul2( h.bt2, tb ); }
+    const R spd_m1 = s0.x - uabs( b_x ) * rs.x, spd_p1 = s0.y + uabs( b_x ) * rs.y;
     // the side the face lies on, and whether outside its fan, in its star or
     // in its double-star region
     const bool out_l = h.spd_m2 >= 0, out_r = h.spd_p2 <= 0, outer = out_l || out_r;
-    const bool left = out_l || ( ! out_r && spd0 >= 0 );
+    const bool left = out_l || ( ! out_r && s0.x >= 0 );
     const bool inner = ! outer && ( left ? spd_m1 < 0 : spd_p1 > 0 ) && bx_2 > flat;
-    R rho = left ? h.rho.x : h.rho.y, vn = left ? h.vn.x : h.vn.y, p = left ? pt.x : pt.y;
+    const R rho = left ? h.rho.x : h.rho.y;
+    R vn = left ? h.vn.x : h.vn.y, p = left ? pt.x : pt.y;
     R v1 = left ? h.vt1.x : h.vt1.y, v2 = left ? h.vt2.x : h.vt2.y;
     R b1 = left ? h.bt1.x : h.bt1.y, bb2 = left ? h.bt2.x : h.bt2.y;
-    const R pre = left ? h.pre.x : h.pre.y, pm = left ? h.pm.x : h.pm.y;
-    R en = pre * e.cv + rho * ( vn * vn + v1 * v1 + v2 * v2 ) * R( 0.5f ) + pm;
+    const R pre = left ? h.pre.x : h.pre.y;
+    const R vv = vn * vn + v1 * v1 + v2 * v2;
+    R en;
+    if constexpr( F32 ) en = ( p + pre * ( e.cv - 1 ) ) + rho * R( 0.5f ) * vv;   // (the magnetic pressure in p)
+    else                en = pre * e.cv + rho * vv * R( 0.5f ) + ( left ? h.pm.x : h.pm.y );
     R vb = vn * b_x + v1 * b1 + v2 * bb2;
-    R x1 = 0, x2 = 0, mass = left ? u_m.x : u_m.y;
+    R x1 = 0, x2 = 0, mass = left ? u_m.x : u_m.y, mn = mass;
     if( ! outer )
     {
-        const R sdl = left ? sd.x : sd.y, il = left ? ism.x : ism.y;
+        const R il = left ? ism.x : ism.y, ws = left ? w.x : w.y, ms = left ? m.x : m.y;
+        const R so = left ? h.spd_m2 : h.spd_p2, sc = left ? s0.x : s0.y;
         const bool flt = left ? flat_l : flat_r;
-        const R dvn = vn - spd0;
-        x1 = flt ? b1 * dvn : R( 0 );
-        x2 = flt ? bb2 * dvn : R( 0 );
-        const R rho_s = left ? rhos.x : rhos.y;
-        if constexpr( sizeof( R ) == 8 )
+        x1 = flt ? - b1 * ws : R( 0 );
+        x2 = flt ? - bb2 * ws : R( 0 );
+        v1 = left ? vs1.x : vs1.y; v2 = left ? vs2.x : vs2.y;
+        b1 = left ? bs1.x : bs1.y; bb2 = left ? bs2.x : bs2.y;
+        const R vbs = sc * b_x + v1 * b1 + v2 * bb2;
+        if constexpr( F32 )
+        {   // rho* - rho = rho ( S_M - v_n ) / ( S - S_M ), E* - E and p* - p alike
+            mass += so * ( rho * ws * il );
+            mn = mass;
+            en += ( b_x * ( vb - vbs ) + ws * ( en + p + ms * sc ) ) * il;
+            p += ms * ws;
+        }
+        else
         {   // FP64: the mass flux as the sum of its jumps.  Against a wall it is
             // rounding residue, whose sign the edge EMF's upwind switch reads:
             // the region's rho S_M is exactly zero there, which the reference's
             // sum is not
-            const R so = left ? h.spd_m2 : h.spd_p2, si = left ? spd_m1 : spd_p1;
+            const R si = left ? spd_m1 : spd_p1, rho_s = left ? rhos.x : rhos.y;
             mass += ( left ? si < 0 : si > 0 ) ? - so * rho - ( si - so ) * rho_s + si * rho_s
                                                : so * ( rho_s - rho );
+            mn = rho_s * sc;
+            en = ( b_x * ( vb - vbs ) - p * vn + ( left ? sd.x : sd.y ) * en + ptot_s * sc ) * il;
+            p = ptot_s;
         }
-        else
-            mass = rho_s * spd0;
-        rho = rho_s;
-        v1 = left ? vs1.x : vs1.y; v2 = left ? vs2.x : vs2.y;
-        b1 = left ? bs1.x : bs1.y; bb2 = left ? bs2.x : bs2.y;
-        const R vbs = spd0 * b_x + v1 * b1 + v2 * bb2;
-        en = ( b_x * ( vb - vbs ) - p * vn + sdl * en + ptot_s * spd0 ) * il;
         vb = vbs;
-        vn = spd0;
-        p = ptot_s;
+        vn = sc;
         if( inner )
         {
             const R sg = b_x > 0 ? R( 1 ) : R( -1 );
             const R rni = rcp( sq.x + sq.y ), ss = sg * sq.x * sq.y;
-            v1 = rni * ( sq.x * vs1.x + sq.y * vs1.y + sg * ( bs1.y - bs1.x ) );
-            v2 = rni * ( sq.x * vs2.x + sq.y * vs2.y + sg * ( bs2.y - bs2.x ) );
-            b1 = rni * ( sq.x * bs1.y + sq.y * bs1.x + ss * ( vs1.y - vs1.x ) );
-            bb2 = rni * ( sq.x * bs2.y + sq.y * bs2.x + ss * ( vs2.y - vs2.x ) );
-            const R vbd = spd0 * b_x + v1 * b1 + v2 * bb2;
+            const R dv1 = vs1.y - vs1.x, dv2 = vs2.y - vs2.x, db1 = bs1.y - bs1.x, db2 = bs2.y - bs2.x;
+            if constexpr( F32 )
+            {   // this side's star state plus the differences' share
+                const R cv = left ? sq.y : - sq.x, cb = left ? sq.x : - sq.y;
+                v1 += rni * ( cv * dv1 + sg * db1 );
+                v2 += rni * ( cv * dv2 + sg * db2 );
+                b1 += rni * ( cb * db1 + ss * dv1 );
+                bb2 += rni * ( cb * db2 + ss * dv2 );
+            }
+            else
+            {
+                v1 = rni * ( sq.x * vs1.x + sq.y * vs1.y + sg * db1 );
+                v2 = rni * ( sq.x * vs2.x + sq.y * vs2.y + sg * db2 );
+                b1 = rni * ( sq.x * bs1.y + sq.y * bs1.x + ss * dv1 );
+                bb2 = rni * ( sq.x * bs2.y + sq.y * bs2.x + ss * dv2 );
+            }
+            const R vbd = sc * b_x + v1 * b1 + v2 * bb2;
             en += ( left ? -sq.x : sq.y ) * sg * ( vb - vbd );
             vb = vbd;
         }
     }
-    const R mn = rho * vn;
     flx[ RHO ] = mass;
     flx[ ENE ] = ( en + p ) * vn - b_x * vb;
     flx[ MOM ] = mn * vn + p - bx_2;
@@ -387,7 +428,7 @@ void hlle_tail( R * flx, const hll_prefix< R > & h, const eos_c< R > & e )
     const R s_l = rmin( h.spd_m2, R( 0 ) );
     const R s_r = rmax( h.spd_p2, R( 0 ) );
     const R inv = rcp( s_r - s_l ), slr = s_r * s_l;
-    const P bx = mk2( h.b_x, h.b_x ), half = mk2( R( 0.5f ), R( 0.5f ) );
+    const P nbx = mk2( -h.b_x, -h.b_x ), half = mk2( R( 0.5f ), R( 0.5f ) );
     const P mn = mul2( h.rho, h.vn );
     const P v2 = mad2( h.vn, h.vn, mad2( h.vt1, h.vt1, mul2( h.vt2, h.vt2 ) ) );
     const P en = mad2( h.pre, mk2( e.cv, e.cv ), mad2( mul2( half, h.rho ), v2, h.pm ) );
@@ -395,13 +436,13 @@ void hlle_tail( R * flx, const hll_prefix< R > & h, const eos_c< R > & e )
     const P vb = mad2( h.vt1, h.bt1, mul2( h.vt2, h.bt2 ) );
     auto join = [ & ]( P f, P u ) { return ( s_r * f.x - s_l * f.y + slr * ( u.y - u.x ) ) * inv; };
     flx[ RHO ] = join( mn, h.rho );
-    flx[ ENE ] = join( sub2( mul2( h.vn, add2( pt, en ) ), mul2( bx, vb ) ), en );
+    flx[ ENE ] = join( mad2( nbx, vb, mul2( h.vn, add2( pt, en ) ) ), en );
     flx[ MOM ] = join( mad2( mn, h.vn, pt ), mn );
-    flx[ MOM + 1 ] = join( sub2( mul2( mn, h.vt1 ), mul2( bx, h.bt1 ) ), mul2( h.rho, h.vt1 ) );
-    flx[ MOM + 2 ] = join( sub2( mul2( mn, h.vt2 ), mul2( bx, h.bt2 ) ), mul2( h.rho, h.vt2 ) );
+    flx[ MOM + 1 ] = join( mad2( nbx, h.bt1, mul2( mn, h.vt1 ) ), mul2( h.rho, h.vt1 ) );
+    flx[ MOM + 2 ] = join( mad2( nbx, h.bt2, mul2( mn, h.vt2 ) ), mul2( h.rho, h.vt2 ) );
     flx[ BCC ] = 0;
-    flx[ BCC + 1 ] = join( sub2( mul2( h.bt1, h.vn ), mul2( bx, h.vt1 ) ), h.bt1 );
-    flx[ BCC + 2 ] = join( sub2( mul2( h.bt2, h.vn ), mul2( bx, h.vt2 ) ), h.bt2 );
+    flx[ BCC + 1 ] = join( mad2( nbx, h.vt1, mul2( h.bt1, h.vn ) ), h.bt1 );
+    flx[ BCC + 2 ] = join( mad2( nbx, h.vt2, mul2( h.bt2, h.vn ) ), h.bt2 );
 }
 
 template< class R > __device__ __forceinline__
