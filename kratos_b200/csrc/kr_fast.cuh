@@ -226,8 +226,8 @@ void hllc_fast( R * flx, const R * wl, const R * wr, const eos_c< R > & e )
 // Flux sweeps z / y / x of the 256^3 mesh in 64 blocks of 64^3, ms per launch, one
 // thread per face, two-sided -> one-sided with the reciprocals above: FP64 1.62 /
 // 1.50 / 1.41 -> 0.67 / 0.65 / 0.58, FP32 0.48 / 0.45 / 0.37 -> 0.35 / 0.33 / 0.31
-// (direct and difference forms alike: 600 / 643 / 704 and 611 / 643 / 708 us per step
-// with the march).
+// (direct and difference forms, us per step with the march: 598 / 643 / 701 and
+// 598 / 643 / 714).
 
 template< class R > struct lr_t;
 template<> struct lr_t< float >  { typedef float2 type; };

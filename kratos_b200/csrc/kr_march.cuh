@@ -29,7 +29,9 @@ __device__ __forceinline__ void cp_async8( void * s, const void * g )
 
 // Lower (q - s) and upper (q + s) states of a cell's 8 words from it and its two
 // neighbours (rings of 16-byte groups, strided by 128); the normal field's word
-// is left out in FP64.  plm_face_fast's and plm_face_fast2's operations.
+// is left out in FP64.  plm_face_fast's and plm_face_fast2's operations; without a
+// slope the cell's own value is selected, so a neighbour that is no number (or a
+// donor's, the VL2 predictor) leaves it alone.
 template< int AXIS > __device__ __forceinline__
 void plm_cell( const float4 * qm, const float4 * q, const float4 * qp, bool donor, float * lo, float * hi )
 {
@@ -46,12 +48,12 @@ void plm_cell( const float4 * qm, const float4 * q, const float4 * qp, bool dono
             const float2 z = h ? make_float2( d.z, d.w ) : make_float2( d.x, d.y );
             const float2 dl = __ffma2_rn( x, m1, y ), dr = __ffma2_rn( y, m1, z );
             const float2 p = __fmul2_rn( dl, dr ), s = __fadd2_rn( dl, dr );
-            float2 t = __fmul2_rn( dr, make_float2( rcp( s.x ), rcp( s.y ) ) );
-            t = make_float2( p.x > 0.f && ! donor ? t.x : 0.f, p.y > 0.f && ! donor ? t.y : 0.f );
+            const float2 t = __fmul2_rn( dr, make_float2( rcp( s.x ), rcp( s.y ) ) );
             const float2 u = __ffma2_rn( dl, t, y ), l = __ffma2_rn( dl, __fmul2_rn( t, m1 ), y );
+            const bool px = p.x > 0.f && ! donor, py = p.y > 0.f && ! donor;
             const int w = 4 * k + 2 * h;
-            lo[ w ] = l.x; lo[ w + 1 ] = l.y;
-            hi[ w ] = u.x; hi[ w + 1 ] = u.y;
+            lo[ w ] = px ? l.x : y.x; lo[ w + 1 ] = py ? l.y : y.y;
+            hi[ w ] = px ? u.x : y.x; hi[ w + 1 ] = py ? u.y : y.y;
         }
     }
 }

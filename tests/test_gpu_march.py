@@ -42,3 +42,25 @@ def test_flat_block(precision):
     d.step(2)
     _check(d, o, n, precision)
     d.close()
+
+
+@pytest.mark.parametrize("integrator", [0, 1])
+def test_not_a_number_spreads_no_further(integrator):
+    """A cell without a velocity (NaN momentum) makes the same cells and faces NaN
+    in the mixed step as in FP64: its neighbours' slopes, which it has a part in,
+    are zero, so their other faces stay numbers."""
+    from kratos_b200 import Dynamics
+    nb, n = (1, 1, 1), (130, 131, 70)
+    u0, b0 = _state(nb, n, "subsonic", 5)
+    u0[0, 30, 60, 61, 3] = np.nan
+    bad = []
+    for precision in (2, 1):
+        d = Dynamics(True, nb, n, gamma=GAMMA, precision=precision, integrator=integrator)
+        d.set_state(u0, b0)
+        d.step(1)
+        u, b = d.get_state()
+        bad.append((np.isnan(u).any(-1), np.isnan(b[:, 2:-2, 2:-2, 2:-2])))
+        d.close()
+    assert 0 < bad[0][0].sum() < 200
+    for k in range(2):
+        assert np.array_equal(bad[0][k], bad[1][k]), (bad[0][k].sum(), bad[1][k].sum())
