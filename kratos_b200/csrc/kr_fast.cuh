@@ -98,7 +98,7 @@ void plm_face_fast( R q_ll, R q_l, R q_r, R q_rr, R & ql, R & qr )
         const bool lpos = dql * dqc > R( 0 );
         const bool rpos = dqr * dqc > R( 0 );
         ql = lpos ? q_l + dql * ( dqc * rcp( dql + dqc ) ) : q_l;
-        qr = rpos ? q_r - dqr * ( dqc * rcp( dqc + dqr ) ) : q_r;
+        qr = rpos ? q_r - dqc * ( dqr * rcp( dqc + dqr ) ) : q_r;
         return;
     }
     ql = q_l + plm_slope( q_ll, q_l, q_r );
@@ -126,6 +126,8 @@ void plm_face_fast2( float2 q_ll, float2 q_l, float2 q_r, float2 q_rr, float2 & 
     const float2 il = make_float2( rcp( sl.x ), rcp( sl.y ) ), ir = make_float2( rcp( sr.x ), rcp( sr.y ) );
     const float2 tl = __fmul2_rn( dqc, il );
     const float2 tr = __fmul2_rn( __fmul2_rn( dqr, ir ), m1 );
+    // a cell's slope is its lower difference times the upper one's share of their
+    // sum, at both of its faces (as the march forms it, once for both)
     const float2 cl = __ffma2_rn( dql, tl, q_l );        // q_l + dql ( dqc / ( dql + dqc ) )
     const float2 cr = __ffma2_rn( dqc, tr, q_r );        // q_r - dqc ( dqr / ( dqc + dqr ) )
     ql = make_float2( lx ? cl.x : q_l.x, ly ? cl.y : q_l.y );
