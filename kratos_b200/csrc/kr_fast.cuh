@@ -20,11 +20,27 @@ template< class R > struct eos_c
     R gamma, gm1, cv;        // gamma, gamma - 1, 1 / (gamma - 1)
 };
 
-// FP32 (the mixed step, whose error budget is 1e-4 in density): the SFU
-// approximations, one MUFU instruction each.  The .ftz forms: without them every
-// reciprocal carries a compare and two scalings for subnormal inputs, which no
-// caller has (densities and pressures are above their floors, the limiter's sums
-// are normal, below).  A subnormal square is taken as zero.
+// Reciprocals and roots without the library functions' branches for zero,
+// subnormal, infinite and NaN arguments, so that a face's independent ones overlap.
+//
+// FP32: the hardware approximations, one instruction each (rcp 1 ulp, rsqrt 2^-22.9
+// relative by the PTX ISA), in their .ftz forms: the others carry a compare and two
+// scalings for subnormal inputs.  Arguments: densities, pressures and differences of
+// wave speeds between 2^-126 and 2^126; a square below FLT_MIN counts as zero (a
+// speed below 1.1e-19 in code units, and in the fast speed's root, which takes
+// fourth powers, one below 3e-10).
+//
+// FP64: Newton-Raphson from the hardware approximations (about 20 bits).
+//  - reciprocal, from f( y ) = 1 / y - x: y += y ( 1 - x y ), twice: 2^-40, 2^-80;
+//    what is left is the last rounding, 2^-53.
+//  - reciprocal root: with e = 1 - x y^2, x^-1/2 = y ( 1 - e )^-1/2 = y ( 1 + e / 2 +
+//    3 e^2 / 8 + ... ) (the binomial series), first to e^2 (5 / 16 e^3 is left, 2^-58),
+//    then to e: the last rounding and half of x y's, 1.5 x 2^-53.
+//  - root: g = x y, then Newton-Raphson on g^2 = x, g += ( x - g^2 ) / ( 2 g ) with
+//    1 / g = y: the last rounding, 2^-53.
+// Arguments: 2^-1021 to 2^1021 in size (positive for the roots); a square below
+// 1e-290 counts as zero; NaN stays NaN; zero and infinity give NaN, and callers
+// select such results away.
 __device__ __forceinline__ float rcp( float x )
 {
     float y;
@@ -38,11 +54,6 @@ __device__ __forceinline__ float rsq( float x )
     return y;
 }
 __device__ __forceinline__ float fsqrt( float x ) { return x >= FLT_MIN ? x * rsq( x ) : 0.f; }
-// FP64: Newton-Raphson from the hardware's approximations (about 20 bits): two
-// steps y += y ( 1 - x y ) of the reciprocal; for the reciprocal root one step of
-// third order, from e = 1 - x y^2: y ( 1 + e / 2 + 3 e^2 / 8 ), and one of second.
-// Without the library functions' branches for zero, subnormal and infinite
-// arguments, a face's independent reciprocals overlap.
 __device__ __forceinline__ double rcp( double x )
 {
     double y;
@@ -63,9 +74,9 @@ __device__ __forceinline__ double rsq( double x )
     return fma( 0.5 * y, fma( -x * y, y, 1.0 ), y );
 }
 __device__ __forceinline__ double fsqrt( double x )
-{   // x / sqrt( x ) with one correction of the product
+{
     const double y = rsq3( x ), g = x * y;
-    return x > 1e-290 ? fma( 0.5 * y, fma( -g, g, x ), g ) : 0.0;
+    return x < 1e-290 ? 0.0 : fma( 0.5 * y, fma( -g, g, x ), g );
 }
 
 // Limited slope of a cell (half its van Leer difference, plm.h:116-153
