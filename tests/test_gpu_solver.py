@@ -19,7 +19,8 @@ FLOWS = {
     # velocity scale, field scale, field along z, spread of log density and pressure
     "subsonic": (0.2, 0.7, 0.3, 0.3),
     "supersonic": (8.0, 0.5, 0.2, 0.5),
-    "no_normal_field": (0.5, 0.0, 0.0, 0.5),
+    "no_normal_field": (0.5, 0.6, 0.0, 0.5),        # none along z, transverse ones on its faces
+    "no_field": (0.5, 0.0, 0.0, 0.5),
     "tiny_normal_field": (0.5, 0.6, 1e-4, 0.5),
     "strong_field": (0.5, 4.0, 2.0, 1.0),
 }
@@ -72,7 +73,10 @@ def test_one_step_from_random_states(nb, n, flow, precision):
         scale = np.abs(uo[..., 2:5]).max(-1).sum() if k >= 2 else np.abs(uo[..., k]).sum()
         assert np.abs(u[..., k] - uo[..., k]).sum() <= tol * scale, "field %d" % k
     own = np.s_[:, 2:n[2] + 2, 2:n[1] + 2, 2:n[0] + 2]
-    assert np.abs(b[own] - bo[own]).sum() <= tol * max(np.abs(bo[own]).sum(), np.abs(u0[..., 0]).sum())
+    if flow == "no_field":
+        assert not b[own].any() and not bo[own].any()
+    else:
+        assert np.abs(b[own] - bo[own]).sum() <= tol * np.abs(bo[own]).sum()
     d.close()
 
 
