@@ -1026,14 +1026,16 @@ void learned_solve( const args_t< R > & a, int b, int axis, const int * ii, bool
 
 // Resident CTAs per SM the per-face sweep is compiled for: register budgets
 // that ptxas meets without spilling (FP32 default / HLLE: 64 registers, 8 CTAs;
-// learned with the network: 6; FP64: 4).  The learned sweep without the network
-// holds both solvers: at 64 registers it spills 12 bytes and still ran 0.5%
-// faster per step than at 72 (7 CTAs).
+// learned with the network: 6; FP64: 96 registers, 5, with the network or the
+// samples 4).  The learned FP32 sweep without the network holds both solvers: at
+// 64 registers it spills 12 bytes and still ran 0.5% faster per step than at 72 (7
+// CTAs).  FP64 left to choose took 104 registers, 4 CTAs: x sweep of 256^3 1270 us
+// per step against 1151.
 template< class R, int MODE > constexpr int flux_min_ctas(  )
 {
     return sizeof( R ) == 4 ? ( ( MODE <= KR_RIEMANN_HLLE || MODE == FLUX_APPLY ) ? 8
                                 : ( MODE == KR_RIEMANN_LEARNED ? 6 : 4 ) )
-                            : ( MODE == KR_RIEMANN_HLLE ? 5 : 4 );
+                            : ( ( MODE <= KR_RIEMANN_HLLE || MODE == FLUX_APPLY ) ? 5 : 4 );
 }
 
 // The normal B of a face for the reconstruction: the face lattice's value;
