@@ -470,6 +470,8 @@ static std::string batch_key( const kr_batch * bt )
         k += ( * p == ' ' ) ? '_' : * p;
     k += " sm" + std::to_string( prop.multiProcessorCount ) + " prec" + std::to_string( bt->precision )
        + " riemann" + std::to_string( bt->riemann );
+    if( bt->march[ 1 ] || bt->march[ 2 ] )   // other kernels: counts tuned for the per-face sweeps don't apply
+        k += " march";
     for( kr_ctx * c : bt->ctx )
         k += " " + std::to_string( c->cfg.n[ 0 ] ) + "x" + std::to_string( c->nblk );
     return k;

@@ -181,3 +181,16 @@ def test_batch_of_long_boxes():
     assert bt, L.lib().kr_batch_last_error(None).decode()
     L.lib().kr_batch_destroy(bt)
     d.close()
+
+
+def test_tuned_counts_of_other_sweeps_are_not_reused(tmp_path):
+    """A cache line of the same boxes tuned where the y and z sweeps ran face by
+    face is no hit for a batch that marches."""
+    from kratos_b200.boxes import BoxBatch
+    cache = tmp_path / "tune.txt"
+    bb = BoxBatch(5, 24, batched=True, precision=1)
+    bb.autotune(str(cache))
+    cache.write_text(cache.read_text().replace(" march", ""))
+    _, cached = bb.autotune(str(cache))
+    assert not cached
+    bb.close()
