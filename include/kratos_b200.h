@@ -291,7 +291,8 @@ int kr_c2p_dt_noalloc( const kr_cfg * cfg, const double * u, const double * bf,
  * as one persistent launch over all their blocks: its CTAs walk a work list of
  * the CTA tiles of every block (bigger blocks first), with the per-group
  * arguments in the kernel's parameter space, and give the per-context steps'
- * results bit for bit.  One CUDA graph per step (14 launches, 20 with the
+ * results to the rounding of the same operations (other kernels: the compiler
+ * may fuse multiply-adds differently).  One CUDA graph per step (14 launches, 20 with the
  * learned selector: stage 0's update and stage 1's c2p fused; 16 and 22 for
  * contexts made with KR_FLAG_UNFUSED), on the first context's stream.  The contexts stay owned
  * by the caller and must outlive the batch; their state, times and selector

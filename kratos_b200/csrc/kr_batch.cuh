@@ -6,9 +6,15 @@
 // (group, block, plane of a sweep, tile), bigger blocks first.  A CTA
 // takes items blockIdx.x, blockIdx.x + gridDim.x, ... and runs the same
 // per-site code on the item's group arguments (read from the kernel's
-// parameter space by the item's group index), so a batched step gives the
-// per-group steps' results bit for bit while 1024 boxes of five sizes step in
-// 14 launches instead of 5 x 14, captured as one CUDA graph.  The list is not
+// parameter space by the item's group index).  1024 boxes of five sizes step in
+// 14 launches instead of 5 x 14, captured as one CUDA graph, and agree with the
+// per-group steps to the rounding of the same operations in other kernels (24
+// boxes, 4 steps, mixed: the conserved words bit for bit, face B to 1e-16; FP64:
+// 1e-16).  Whether the y and z sweeps march is the whole batch's choice.  The
+// kinds run one after the other with a tail each, where the per-size graphs
+// overlap on their streams, so on one GPU the batch is the slower of the two:
+// 256 boxes, mixed 7.1 ms per step against 5.9, FP64 10.5 against 9.4; 1024,
+// mixed 33.3 (31.7 tuned) against 26.9.  What it saves is launches.  The list is not
 // stored: an item is decoded from its number with the list's per-group
 // offsets and extents (batch_item), so the group index -- and every argument
 // read through it -- is the same for all threads of the CTA and the compiler
@@ -44,7 +50,7 @@ struct multi_t
     udiv_t l_planes[ KR_BATCH_LISTS ][ KR_BATCH_MAX ];
 };
 
-// Item it of work list `list`: x group, y block, z plane, w tile.  Uniform over
+// Item it of work list `list`: x group, y block, z plane of the list, w tile.  Uniform over
 // the CTA when it is (it comes from blockIdx and the loop counter).
 template< class R > __device__ __forceinline__
 int4 batch_item( const multi_t< R > & m, int list, int it )
@@ -80,7 +86,7 @@ __global__ void k_step_end_multi( const __grid_constant__ multi_scal_t m, double
         step_end( m.s[ g ], dt_expand, m.ns[ g ] );
 }
 
-// item: x group, y block, z plane, w tile
+// item: x group, y block, z plane of the list, w tile
 template< bool MHD, class R, bool DT >
 __global__ void __launch_bounds__( 256, ( MHD && DT ) ? 3 : 4 )
 k_c2p_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
@@ -165,7 +171,7 @@ k_update_list( const __grid_constant__ multi_t< R > m, int step, int n_items )
 }
 
 // Stage 0's update, CT and stage 1's c2p in one launch (update_c2p_cell), over
-// the c2p work list (item: x group, y block, z plane, w tile of 256 cells).
+// the cells' work list (item: x group, y block, w tile of 256 cells).
 template< class R >
 __global__ void __launch_bounds__( 256, 3 )
 k_update_c2p_list( const __grid_constant__ multi_t< R > m, int n_items )
@@ -182,7 +188,10 @@ k_update_c2p_list( const __grid_constant__ multi_t< R > m, int n_items )
 // Launch kinds with a tunable grid, in this order in kr_batch::grid.
 enum { BK_C2P0, BK_C2P1, BK_FLUX, BK_EVAL, BK_EMF, BK_UPD1, BK_UPD2, BK_UPDC2P, BK_N };
 static const char * const BK_NAME[ BK_N ] = { "c2p0", "c2p1", "flux", "eval", "emf", "upd1", "upd2", "updc2p" };
-// resident CTAs per SM each kind is compiled for (its __launch_bounds__)
+// resident CTAs per SM each kind is compiled for (its __launch_bounds__).  The
+// sweeps' is the per-face kernel's, also where the y and z sweeps march (with the
+// march's own count, 3/4 of it in FP32, 256 boxes took 7.16 ms against 7.13, 1024
+// 34.1 against 33.3).
 template< class R > static int bk_min_ctas( int k )
 {
     switch( k )

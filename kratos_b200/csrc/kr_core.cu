@@ -1027,9 +1027,8 @@ void learned_solve( const args_t< R > & a, int b, int axis, const int * ii, bool
 // Resident CTAs per SM the per-face sweep is compiled for: register budgets
 // that ptxas meets without spilling (FP32 default / HLLE: 64 registers, 8 CTAs;
 // learned with the network: 6; FP64: 96 registers, 5, with the network or the
-// samples 4).  The learned FP32 sweep without the network holds both solvers: at
-// 64 registers it spills 12 bytes and still ran 0.5% faster per step than at 72 (7
-// CTAs).  FP64 left to choose took 104 registers, 4 CTAs: x sweep of 256^3 1270 us
+// samples 4).  The learned FP32 sweep without the network holds both solvers, 60
+// registers.  FP64 left to choose took 104 registers, 4 CTAs: x sweep of 256^3 1270 us
 // per step against 1151.
 template< class R, int MODE > constexpr int flux_min_ctas(  )
 {
@@ -1221,7 +1220,7 @@ __global__ void __launch_bounds__( 128, ( flux_min_ctas< R, MODE >(  ) ) ) k_flu
     bool hlle_warp = false;
     if constexpr( MODE == FLUX_APPLY )
     {   // learned mode, sweeps without the network: this warp's solver choice,
-        // loaded first (gridDim.x: 128-face chunks per z plane)
+        // loaded first (gridDim.x: 128-face chunks per plane, face_plane_axis)
         if( step == 0 && sel_eval_step( a.s, a.sel_period ) )
             return;                   // the network's sweep (k_flux_eval) solves this one
         hlle_warp = ( a.sel_dec[ ( ( size_t ) axis * a.nblk + blockIdx.z ) * a.sel_wcap
@@ -1232,7 +1231,7 @@ __global__ void __launch_bounds__( 128, ( flux_min_ctas< R, MODE >(  ) ) ) k_flu
 }
 
 // Learned mode, the network's sweep: a fixed grid strides over the 128-face
-// chunks (cpp per z plane, nz planes), so on the stages where the network does
+// chunks (cpp per plane of face_plane_axis, nz planes), so on the stages where the network does
 // not run (k_flux<FLUX_APPLY> solves them) only this small grid launches and
 // exits.
 template< bool MHD, class R, int AXIS >
@@ -2856,9 +2855,6 @@ static kr_ctx * create_ctx( const kr_cfg * cfg, int n_regions, const kr_region *
     c->cfg = * cfg;
     c->n_sm = n_sm;
     c->boxes = ( cfg->flags & KR_FLAG_BOXES ) != 0;
-    // The shared-memory tiled sweep is opt-in: on the 256^3 OT step it measured
-    // slower than the per-face kernel (more registers per thread, long per-thread
-    // face loops, a tail of partial CTAs), so the per-face kernel is the default.
     const int * n = cfg->n;
     c->nranks = ranks_of( * cfg );
     c->rank = c->nranks > 1 ? cfg->rank : 0;
@@ -2999,8 +2995,8 @@ static kr_ctx * create_ctx( const kr_cfg * cfg, int n_regions, const kr_region *
                 && ck( c, cudaMalloc( & c->sel_cnt, 2 * sizeof( unsigned long long ) ), "malloc selector" )
                 && ck( c, cudaMemset( c->sel_cnt, 0, 2 * sizeof( unsigned long long ) ), "memset selector" );
     if( cfg->mhd && cfg->riemann == KR_RIEMANN_LEARNED && ok )
-    {   // per (axis, block): one byte per warp of the per-face sweep's grid
-        // (128-face chunks per z plane x z planes x 4 warps)
+    {   // per (axis, block): one 32-bit mask of choices per warp of the sweep's
+        // faces (128-face chunks per plane of face_plane_axis x planes x 4 warps)
         for( int ax = 0; ax < 3; ++ ax )
         {
             long long ext[ 3 ];

@@ -229,9 +229,9 @@ static inline march_t march_shape( const int * n, int axis, long long nblk, int 
     return s;
 }
 
-// Whether blocks n march along y and z: at least a wave of warps (32 per SM) with
-// eight faces each; smaller meshes need k_flux's one thread per face to fill the
-// chip.  The mesh's own block count, not a rank's, so that every rank of a
+// Whether blocks n march along y and z: at least 32 warps per SM with eight faces
+// each (24 are resident in FP32, 16 in FP64); smaller meshes need k_flux's one
+// thread per face to fill the chip.  The mesh's own block count, not a rank's, so that every rank of a
 // sharded mesh and an unsharded one run the same kernels.  Measured per step, load
 // over the line, k_flux -> march: 1.87 (8 blocks of 64^3) FP32 659 -> 639 us, FP64
 // 987 -> 969; 1.80 (one block of 128^3) FP32 620 -> 598, FP64 934 -> 905.  With the

@@ -104,8 +104,7 @@ int c2p( const double * cons_in, double * prim, double * cons_out, double gamma,
 
 ////////////////////////////////////////////////////////////
 // Physical flux of a rotated hydro state (hydro/riemann/hllc.h:239-250
-// f_lr_hyd) and of an MHD state (mhd/riemann/hlld.h:49-80 f_flux), used by
-// the solvers in kr_fast.cuh.
+// f_lr_hyd), used by the solver in kr_fast.cuh.
 
 template< class R > __device__ __forceinline__
 void f_lr_hyd( R * f, const R * w, R v, R e )
@@ -117,20 +116,6 @@ void f_lr_hyd( R * f, const R * w, R v, R e )
     for( int a = MOM; a < MOM + 3; ++ a )
         f[ a ] = rho * w[ a ] * v;
     f[ MOM ] += pre;
-}
-
-template< class R > __device__ __forceinline__
-void hlld_f_flux( R * flux, const R * u, const R * w, R p_tot, R b_x )
-{
-    const R bx_2 = b_x * b_x;
-    flux[ RHO ] = u[ MOM ];
-    flux[ ENE ] = w[ MOM ] * ( p_tot + u[ ENE ] - bx_2 ) - b_x
-                * ( w[ MOM + 1 ] * u[ BCC + 1 ] + w[ MOM + 2 ] * u[ BCC + 2 ] );
-    flux[ MOM ]     = p_tot - bx_2 + u[ MOM ] * w[ MOM ];
-    flux[ MOM + 1 ] = -b_x * u[ BCC + 1 ] + u[ MOM + 1 ] * w[ MOM ];
-    flux[ MOM + 2 ] = -b_x * u[ BCC + 2 ] + u[ MOM + 2 ] * w[ MOM ];
-    flux[ BCC + 1 ] = -b_x * w[ MOM + 1 ] + u[ BCC + 1 ] * w[ MOM ];
-    flux[ BCC + 2 ] = -b_x * w[ MOM + 2 ] + u[ BCC + 2 ] * w[ MOM ];
 }
 
 }   // namespace kr

@@ -102,8 +102,8 @@ def test_batched_launch_matches_per_group_launches(kw):
     grid of one wave, the boxes' states, times and dt agree with the per-group
     steps to the rounding of the step's arithmetic (FP64: 1e-12 relative;
     mixed and learned: 1e-6, the learned mode's HLLE choices within 1% of the
-    faces).  Measured: bit for bit in FP64 and the learned mode, rounding-level
-    differences in the mixed mode."""
+    faces).  Measured: density within 8e-17 in FP64, the conserved words bit for bit
+    in the mixed and learned modes, face B to its last bits in all."""
     from kratos_b200.boxes import BoxBatch
     from kratos_b200 import selector as S
     w = S.init_params(5) if kw.get("riemann") == 2 else None
