@@ -39,12 +39,12 @@ BYTES_PER_ZONE_CYCLE = 320
 # the transverse ghost lines the edge EMF reads: (n+1) ((n+2)^2 - 4) per block.
 FLUX_BYTES_PER_FACE = {4: 8 * 4 + 8 + 7 * 4, 8: 8 * 8 + 8 + 7 * 8}
 # DRAM bytes per face of one FP32 flux launch, ncu dram__bytes_read.sum +
-# dram__bytes_write.sum on this workload (three launches of the first timed
-# step, 1319.3 MB on average) divided by its 18.1 M faces
-FLUX_DRAM_BYTES_PER_FACE = 72.9
+# dram__bytes_write.sum on this workload (the six sweeps of the first timed
+# step, 1347.2 MB on average) divided by its 18.1 M faces
+FLUX_DRAM_BYTES_PER_FACE = 74.4
 # DRAM bytes per zone-cycle of one whole mixed step, ncu on this workload, one
 # kernel kind per capture (profiles/step_dram_mixed_ot256.md)
-STEP_DRAM_BYTES_PER_ZONE_CYCLE_MIXED = 1343.2
+STEP_DRAM_BYTES_PER_ZONE_CYCLE_MIXED = 1330.6
 WORKLOAD = "ot 256^3 periodic MHD, 64 blocks of 64^3, PLM+HLLD+CT, Heun RK2"
 
 
