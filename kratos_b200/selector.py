@@ -99,7 +99,7 @@ def shuffle(X, y, seed=0):
 # a face that a neighbouring block computes too follows its own logit.  On the
 # 256^3 OT mesh (64 blocks of 64^3) that was 28% of the faces, at 6.4e-6 relative
 # L1 density error vs the FP64 step after 45 steps (all-HLLE: 5e-5).  The share is
-# the training's: four seeds gave 14% to 25% on 128^3, and 19% to 47% on Mach 5
+# the training's: four seeds gave 14% to 25% on 128^3, and 19% to 52% on Mach 5
 # turbulence.
 DEFAULT_TOL = 3e-4
 DEFAULT_THRESHOLD = 2.0
